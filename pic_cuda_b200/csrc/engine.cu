@@ -176,6 +176,13 @@ int event_capacity(const pic_job_config& c) {
   return (int)std::max<int64_t>(16384, std::min<int64_t>(ce / 128, 1 << 24));
 }
 
+// FP64 partial sums of a job's level-0 launches: per init tile r^2, F^2 (pairs) and the charge, or a
+// pair per strip item of the level-0 up kernel (at most: the narrowest strips, the shortest rows).
+int64_t partials_bytes(int n) {
+  const int64_t t = (n + 31) / 32;
+  return std::max<int64_t>(24 * t * t, 16ll * mg_up_strips(kMaxFastNu, 0, n) * ((n + 7) / 8));
+}
+
 struct Layout {  // byte sizes of one job's device state
   int levels, lc;
   int nl[PIC_MAX_LEVELS];
@@ -212,7 +219,7 @@ Layout job_layout(const pic_job_config& c, int cluster_C = 0, int cluster_top = 
   for (int l = 1; l < L.levels; ++l) b += 4ll * mgt::round4(L.nl[l]) * L.nl[l];   // up-leg corrections
   b += 4ll * mgt::round4(c.nx) * c.ny;                                           // second level-0 rhs
   b += (int64_t)sizeof(CUtensorMap) * mgt::kTmapsPerLevel * L.levels;
-  b += 24ll * L.ntiles0;
+  b += partials_bytes(c.nx);
   const int64_t ncells = (int64_t)(c.nx - 1) * (c.ny - 1) + 1;
   for (int s = 0; s < c.n_species; ++s) {
     const int64_t cap = round_up(std::max<int64_t>(c.species[s].capacity, 1), PIC_CHUNK);
@@ -420,6 +427,28 @@ void free_job(pic_engine* E, JobHost& J) {
   J.alive = false;
 }
 
+// Rows per strip item of level l for all jobs of a launch, 0 where the tile kernels take the level.
+// An item is one warp, so a level needs about nine of them per SM to hide their latency chains
+// (twelve on the level-0 up kernel, whose tiles are better at 1025^2), and the largest row count
+// that still gives as many wastes least on the rows a strip recomputes before its first; beyond 72
+// rows the last wave costs more than that saves.  Measured on B200, V-cycle with strips against
+// tiles: 4097^2 277 / 401 us, 2049^2 121 / 139, 1025^2 62.6 / 63.3 (66.9 with the level-0 up as
+// strips too); forced at 513^2 67 / 46.5.  Rows per down item at 4097^2: 14 307 us, 30 301, 46 297,
+// 62 297, 94 300, 190 303; per level-0 up item: 12 338, 24 304, 48 289, 72 285, 96 294.
+template <class F>
+int strip_rows(pic_engine* E, const std::vector<int>& ids, int l, F strips, int leg, int nu) {
+  const int per_sm = leg == 1 && l == 0 ? 12 : 9;
+  for (int rows = mg_strip_rows(leg, nu, l, 72); rows > 0; rows = mg_strip_rows(leg, nu, l, rows - 1)) {
+    int64_t items = 0;
+    for (int id : ids) {
+      const JobDev& D = E->jobs[id].dev;
+      if (l < D.lc) items += (int64_t)strips(D.nl[l]) * ((D.nl[l] + rows - 1) / rows);
+    }
+    if (items >= (int64_t)per_sm * E->num_sms) return rows;
+  }
+  return 0;
+}
+
 // Tile lists for the multigrid kernels over the given jobs.
 int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   out.release();
@@ -444,7 +473,6 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
     if (D.lc == 0)
       for (int tj = 0; tj < t0; ++tj)
         for (int ti = 0; ti < t0; ++ti) upd.push_back({id, ti, tj, tj * t0 + ti, t0 * t0, 0});
-    if (D.lc >= 1) finish.push_back(id);
     for (int l = 0; l < D.lc; ++l) {
       const int tc = (D.nl[l + 1] + 15) / 16;
       for (int tj = 0; tj < tc; ++tj)
@@ -461,12 +489,42 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
       coarse_smem = std::max(coarse_smem, mg_coarse_smem(D.nl, D.lc, D.levels));
     }
   }
+  const int fast_pre = (!ids.empty() && nu_pre_min == nu_pre_max && nu_pre_max <= kMaxFastNu) ? nu_pre_max : -1;
+  const int fast_post = (!ids.empty() && nu_post_min == nu_post_max && nu_post_max <= kMaxFastNu) ? nu_post_max : -1;
+  std::vector<TileRef> sdown[PIC_MAX_LEVELS], sup[PIC_MAX_LEVELS];
+  int rows_down[PIC_MAX_LEVELS] = {}, rows_up[PIC_MAX_LEVELS] = {};
+  for (int l = 0; l < max_depth; ++l)
+    for (int leg = 0; leg < 2; ++leg) {
+      const int nu = leg == 0 ? fast_pre : fast_post;
+      if (nu < 0) continue;
+      auto strips = [&](int n) { return leg == 0 ? mg_down_strips(nu, n) : mg_up_strips(nu, l, n); };
+      const int rows = strip_rows(E, ids, l, strips, leg, nu);
+      (leg == 0 ? rows_down : rows_up)[l] = rows;
+      for (int id : ids) {
+        const JobDev& D = E->jobs[id].dev;
+        if (l >= D.lc) continue;
+        const int n = D.nl[l];
+        if (rows == 0) {   // tile kernels
+          const int tu = (n + 31) / 32;
+          if (l == 0 && leg == 1) { finish.push_back(id); finish.push_back(tu * tu); }
+          continue;
+        }
+        const int ts = strips(n), tr = (n + rows - 1) / rows;
+        for (int tj = 0; tj < tr; ++tj)
+          for (int ti = 0; ti < ts; ++ti)
+            (leg == 0 ? sdown : sup)[l].push_back({id, ti, tj, tj * ts + ti, tr * ts, 0});
+        if (l == 0 && leg == 1) { finish.push_back(id); finish.push_back(tr * ts); }
+      }
+    }
   std::vector<TileRef> all;
   size_t off_init = all.size(); all.insert(all.end(), init.begin(), init.end());
   size_t off_upd = all.size(); all.insert(all.end(), upd.begin(), upd.end());
   size_t off_down[PIC_MAX_LEVELS], off_up[PIC_MAX_LEVELS];
   for (int l = 0; l < PIC_MAX_LEVELS; ++l) { off_down[l] = all.size(); all.insert(all.end(), down[l].begin(), down[l].end()); }
   for (int l = 0; l < PIC_MAX_LEVELS; ++l) { off_up[l] = all.size(); all.insert(all.end(), up[l].begin(), up[l].end()); }
+  size_t off_sd[PIC_MAX_LEVELS], off_su[PIC_MAX_LEVELS];
+  for (int l = 0; l < PIC_MAX_LEVELS; ++l) { off_sd[l] = all.size(); all.insert(all.end(), sdown[l].begin(), sdown[l].end()); }
+  for (int l = 0; l < PIC_MAX_LEVELS; ++l) { off_su[l] = all.size(); all.insert(all.end(), sup[l].begin(), sup[l].end()); }
   if (!all.empty()) {
     CK(cudaMalloc(&out.d_tiles, all.size() * sizeof(TileRef)));
     CK(cudaMemcpy(out.d_tiles, all.data(), all.size() * sizeof(TileRef), cudaMemcpyHostToDevice));
@@ -486,10 +544,12 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   for (int l = 0; l < PIC_MAX_LEVELS; ++l) {
     M.down_tiles[l] = out.d_tiles + off_down[l]; M.n_down[l] = (int)down[l].size();
     M.up_tiles[l] = out.d_tiles + off_up[l]; M.n_up[l] = (int)up[l].size();
+    M.down_items[l] = out.d_tiles + off_sd[l]; M.n_down_items[l] = (int)sdown[l].size(); M.down_rows[l] = rows_down[l];
+    M.up_items[l] = out.d_tiles + off_su[l]; M.n_up_items[l] = (int)sup[l].size(); M.up_rows[l] = rows_up[l];
   }
   M.coarse_jobs = out.d_coarse; M.n_coarse = (int)coarse.size();
   M.cluster_jobs = out.d_coarse + coarse.size(); M.n_cluster = (int)cluster.size();
-  M.finish_jobs = out.d_coarse + coarse.size() + cluster.size(); M.n_finish = (int)finish.size();
+  M.finish_jobs = out.d_coarse + coarse.size() + cluster.size(); M.n_finish = (int)finish.size() / 2;
   M.init_jobs = M.finish_jobs + finish.size(); M.n_init_jobs = (int)ids.size();
   M.cluster_C = E->cluster_C;
   M.cluster_smem = cluster_smem;
@@ -499,8 +559,8 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   M.nu_post_max = nu_post_max;
   M.pdl = E->pdl ? 1 : 0;
   M.wide_factor = E->wide_factor;
-  M.fast_nu_pre = (!ids.empty() && nu_pre_min == nu_pre_max) ? nu_pre_max : -1;
-  M.fast_nu_post = (!ids.empty() && nu_post_min == nu_post_max) ? nu_post_max : -1;
+  M.fast_nu_pre = fast_pre;
+  M.fast_nu_post = fast_post;
   // Levels 1..lc as phases of one cooperative launch (PIC_OPT_MG_LEVELS_KERNEL).  Measured on
   // B200 (1025^2 job, CUDA-graph step): 1.600 ms per step against 1.555 ms with one launch per
   // level, because at these sizes each phase waits on its slowest tile either way and the grid
@@ -1064,7 +1124,7 @@ int pic_job_create(pic_engine* E, const pic_job_config* cfg, int* job_id) {
     if (rc) { free_job(E, J); return rc; }
     D.tmaps = tm;
   }
-  ALLOC(D.partials, 24ll * lay.ntiles0);   // per level-0 tile: r^2, F^2 (pairs), then charge
+  ALLOC(D.partials, partials_bytes(c.nx));
   if (c.n_walls > 0) {
     std::vector<double> w(4 * c.n_walls);
     for (int k = 0; k < c.n_walls; ++k) {

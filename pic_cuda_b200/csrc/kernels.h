@@ -69,7 +69,10 @@ struct MgLaunch {
   const TileRef* upd_tiles; int n_upd;                   // level-0 update for jobs with lc == 0
   const int* coarse_jobs; int n_coarse;                  // single-CTA coarse solve
   const int* cluster_jobs; int n_cluster;                // thread-block-cluster coarse solve
-  const int* finish_jobs; int n_finish;                  // jobs with level-0 up tiles (lc >= 1)
+  // strip items (mg_strips.cuh) and their rows per level, empty where the tile kernels take it
+  const TileRef* down_items[PIC_MAX_LEVELS]; int n_down_items[PIC_MAX_LEVELS]; int down_rows[PIC_MAX_LEVELS];
+  const TileRef* up_items[PIC_MAX_LEVELS]; int n_up_items[PIC_MAX_LEVELS]; int up_rows[PIC_MAX_LEVELS];
+  const int* finish_jobs; int n_finish;                  // (job, level-0 partials) of the jobs with lc >= 1
   int cluster_C;
   size_t cluster_smem;
   int max_depth;                                         // max lc over jobs
@@ -92,6 +95,13 @@ struct MgLevelsArgs {
   JobState* st;
   unsigned* gbar;
 };
+// Largest smoothing count of the kernels with compile-time shapes.
+constexpr int kMaxFastNu = 4;
+// Strip layout (mg_strips.cuh): strips across a level of side n, and the most rows per item, at most
+// `at_most`, that fill whole unrolled steps of the kernel (leg 0: down, 1: up; 0 if none does).
+int mg_down_strips(int nu, int n);
+int mg_up_strips(int nu, int level, int n);
+int mg_strip_rows(int leg, int nu, int level, int at_most);
 // Grid size (0: not available) and shared memory of the cooperative levels kernel.
 int mg_levels_configure(int num_sms, int nu_pre_max, int nu_post_max, size_t coarse_smem, size_t* smem,
                         size_t* quarter_floats);

@@ -15,6 +15,8 @@
 //              coarse nodes (fine tile + halo 2*nu+2 in shared memory, every sweep done
 //              locally: a node at distance d from the tile edge is exact for d half-sweeps),
 //              then residual + full weighting straight from shared memory
+//   On levels with enough nodes (strip_rows, engine.cu) both legs run as pipelines of rows in
+//   registers instead of tiles (mg_strips.cuh), with the same bits.
 //   mg_coarse  one CTA per job runs the whole V-cycle from <= 65x65 down in shared memory
 //   (opt-in: levels up to 257^2 or 513^2 in one thread-block cluster, mg_cluster.cu)
 //   mg_up      prolongation + nu_post sweeps on 32x32 tiles; on level 0 also the FP64
@@ -25,6 +27,7 @@
 #include <algorithm>
 #include "common.cuh"
 #include "kernels.h"
+#include "mg_strips.cuh"
 #include "mg_tiles.h"
 #include "tma.cuh"
 
@@ -800,7 +803,6 @@ __global__ void __launch_bounds__(256) mg_up_kernel(const TileRef* __restrict__ 
 // CTA: 256 where a level has enough tiles to fill the GPU, 1024 on small levels, where a
 // tile's latency chain (not the SM's issue rate) sets the time.  Results equal those of
 // mg_down_kernel / mg_up_kernel: the same expressions in the same order at every node.
-constexpr int kMaxFastNu = 4;
 
 // NU red-black SOR sweeps on a W x W tile.  ZERO: the correction enters as 0 (pre-smoothing
 // from a zero guess), so the first half-sweep reads no neighbours (they are all +0).
@@ -1087,11 +1089,10 @@ __global__ void __launch_bounds__(NT, MODE ? 5 : 1) mg_up_fast_kernel(const Tile
       const int q = (oy + 1) * PW + (ox + 1);
       const double rv = rho.mode == 0 ? (double)reinterpret_cast<const float*>(RH)[k]
                         : rho.mode == 1 ? (double)reinterpret_cast<const long long*>(RH)[k] * 0x1p-40 : RH[k];
-      const double F = rhs_scale * rv;
       double r = 0.0;
       if (gx > 0 && gx < nf - 1 && gy > 0 && gy < nf - 1) {
-        const double lap = (P64[q - PW] + P64[q + PW] + P64[q - 1] + P64[q + 1] - 4.0 * P64[q]) * inv_h2;
-        r = F - lap;
+        const double lap = P64[q - PW] + P64[q + PW] + P64[q - 1] + P64[q + 1] - 4.0 * P64[q];
+        r = mgs::defect(lap, inv_h2, rhs_scale, rv, gy);
       }
       pn[g] = P64[q];
       f0[gy * pf + gx] = (float)r;
@@ -1104,8 +1105,9 @@ __global__ void __launch_bounds__(NT, MODE ? 5 : 1) mg_up_fast_kernel(const Tile
   }
 }
 
-// End of a V-cycle for the jobs whose level 0 ran in mg_up_fast_kernel<., 1, .>: one
-// 1024-thread CTA per job sums the tiles' partial norms in a fixed order, counts the cycle,
+// End of a V-cycle for the jobs whose level 0 ran in mg_up_fast_kernel<., 1, .> or
+// mg_up_strip_kernel<., 1>: one
+// 1024-thread CTA per job sums their partial norms in a fixed order, counts the cycle,
 // swaps the potential and defect buffers and takes a converged job out of the running count.  Launched after the
 // level-0 up kernel (waits for it in tma::pdl_wait); the next V-cycle's first launch waits for
 // this one.
@@ -1114,12 +1116,11 @@ __global__ void __launch_bounds__(1024) mg_finish_kernel(const int* __restrict__
                                                         JobState* __restrict__ st, int* running) {
   tma::pdl_trigger();
   tma::pdl_wait();
-  const int job = job_list[blockIdx.x];
+  const int job = job_list[2 * blockIdx.x], n = job_list[2 * blockIdx.x + 1];
   const JobDev& J = jobs[job];
   JobState& T = st[job];
   if (T.converged) return;
-  const int tu = (J.nl[0] + kTU - 1) / kTU;
-  const double r2 = ordered_sum(J.partials, tu * tu, 2, 0);
+  const double r2 = ordered_sum(J.partials, n, 2, 0);
   if (threadIdx.x != 0) return;
   T.rnorm2 = r2;
   T.relres = T.fnorm2 > 0.0 ? sqrt(r2 / T.fnorm2) : sqrt(r2);
@@ -1180,6 +1181,19 @@ void up_fast(int nu, int grid, bool wide, bool pdl, const TileRef* tiles, const 
     case 3: launch_up_fast<3>(grid, wide, pdl, tiles, jobs, st, l, mode, s); break;
     default: launch_up_fast<4>(grid, wide, pdl, tiles, jobs, st, l, mode, s); break;
   }
+}
+
+// Strip launches of one level for the sweep count every job of the launch shares.
+template <int NU>
+void down_strips(int n_items, const TileRef* items, bool pdl, const EngineLaunch& L, int l, int rows, cudaStream_t s) {
+  launch_k(mgs::mg_down_strip_kernel<NU>, (n_items + mgs::kWarps - 1) / mgs::kWarps, 32 * mgs::kWarps, 0, pdl, s, items,
+           n_items, L.jobs, (const JobState*)L.st, l, rows);
+}
+template <int NU>
+void up_strips(int n_items, const TileRef* items, bool pdl, const EngineLaunch& L, int l, int rows, cudaStream_t s) {
+  const int grid = (n_items + mgs::kWarps - 1) / mgs::kWarps;
+  if (l == 0) launch_k(mgs::mg_up_strip_kernel<NU, 1>, grid, 32 * mgs::kWarps, 0, pdl, s, items, n_items, L.jobs, L.st, l, rows);
+  else launch_k(mgs::mg_up_strip_kernel<NU, 0>, grid, 32 * mgs::kWarps, 0, pdl, s, items, n_items, L.jobs, L.st, l, rows);
 }
 
 // ---------------------------------------------------------------- levels 1 .. lc in one launch
@@ -1285,32 +1299,48 @@ int mg_levels_configure(int num_sms, int nu_pre_max, int nu_post_max, size_t coa
   return b >= 1 ? num_sms : 0;  // one CTA per SM
 }
 
-// Tile launches of one level: the compile-time-shape kernels when every job of the launch
-// has the same smoothing count (<= kMaxFastNu), else the generic ones.
-// 1024-thread CTAs where a level has at most wide_factor (default 2) tiles per SM.  pdl: the
-// launch follows a
-// kernel of the V-cycle that this one's prologue may overlap (programmatic serialisation).
+int mg_down_strips(int nu, int n) { return mgs::down_strips(nu, n); }
+int mg_up_strips(int nu, int level, int n) { return mgs::up_strips(nu, level == 0 ? 1 : 0, n); }
+int mg_strip_rows(int leg, int nu, int level, int at_most) { return mgs::rows_fit(leg, nu, level == 0 ? 1 : 0, at_most); }
+
+
+// Launch of one level.  When every job of the launch has the same smoothing count (<= kMaxFastNu):
+// the strip kernels where the level has enough items for them (strip_rows in engine.cu), else the
+// compile-time-shape tile kernels, on 1024-thread CTAs where a level has at most wide_factor
+// (default 2) tiles per SM.  Otherwise the generic tile kernels.  pdl: the launch follows a kernel
+// of the V-cycle that this one's prologue may overlap (programmatic serialisation).
 static bool launch_down(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, cudaStream_t s) {
-  if (M.fast_nu_pre >= 0 && M.fast_nu_pre <= kMaxFastNu) {
+  if (M.n_down_items[l]) {
+    auto* f = M.fast_nu_pre == 0 ? down_strips<0> : M.fast_nu_pre == 1 ? down_strips<1> : M.fast_nu_pre == 2 ? down_strips<2>
+              : M.fast_nu_pre == 3 ? down_strips<3> : down_strips<4>;
+    f(M.n_down_items[l], M.down_items[l], pdl && M.pdl, L, l, M.down_rows[l], s);
+    return true;
+  }
+  if (M.fast_nu_pre >= 0) {
     down_fast(M.fast_nu_pre, M.n_down[l], M.n_down[l] <= M.wide_factor * L.num_sms, pdl && M.pdl, M.down_tiles[l],
-              L.jobs, L.st,
-              l, s);
+              L.jobs, L.st, l, s);
     return true;
   }
   mg_down_kernel<<<M.n_down[l], 256, down_smem(M.nu_pre_max), s>>>(M.down_tiles[l], L.jobs, L.st, l);
   return false;
 }
 static bool launch_up(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, cudaStream_t s) {
-  if (M.fast_nu_post >= 0 && M.fast_nu_post <= kMaxFastNu) {
+  if (M.fast_nu_post < 0) {
+    mg_up_kernel<<<M.n_up[l], 256, up_smem(M.nu_post_max), s>>>(M.up_tiles[l], L.jobs, L.st, l, l == 0 ? 1 : 0,
+                                                                L.running);
+    return false;
+  }
+  if (M.n_up_items[l]) {
+    auto* f = M.fast_nu_post == 0 ? up_strips<0> : M.fast_nu_post == 1 ? up_strips<1> : M.fast_nu_post == 2 ? up_strips<2>
+              : M.fast_nu_post == 3 ? up_strips<3> : up_strips<4>;
+    f(M.n_up_items[l], M.up_items[l], pdl && M.pdl, L, l, M.up_rows[l], s);
+  } else {
     up_fast(M.fast_nu_post, M.n_up[l], M.n_up[l] <= M.wide_factor * L.num_sms, pdl && M.pdl, M.up_tiles[l], L.jobs,
             L.st, l, l == 0 ? 1 : 0, s);
-    if (l == 0)
-      launch_k(mg_finish_kernel, M.n_finish, 1024, 0, M.pdl != 0, s, M.finish_jobs, L.jobs, L.st, L.running);
-    return true;
   }
-  mg_up_kernel<<<M.n_up[l], 256, up_smem(M.nu_post_max), s>>>(M.up_tiles[l], L.jobs, L.st, l, l == 0 ? 1 : 0,
-                                                              L.running);
-  return false;
+  if (l == 0)
+    launch_k(mg_finish_kernel, M.n_finish, 1024, 0, M.pdl != 0, s, M.finish_jobs, L.jobs, L.st, L.running);
+  return true;
 }
 
 int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, cudaStream_t s) {

@@ -72,6 +72,12 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
+// Closes this thread's current group of cp.async copies; waits until at most N of its groups are
+// still in flight (the thread may then read what it copied in the others).
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // Programmatic dependent launch.  A kernel launched with programmatic stream serialisation may
 // start while its predecessor in the stream is still running: it must call pdl_wait() before
 // reading anything the predecessor writes.  pdl_trigger() lets the successor launch once every
