@@ -27,9 +27,11 @@ constexpr int kSortDisorderShift = 5;
 #define PIC_COARSE_MAX 129          // largest level side the one-CTA coarse solver takes (smem)
 #endif
 #ifndef PIC_CHUNK
-#define PIC_CHUNK 512               // particles per mover work item (256 threads x 2)
+#define PIC_CHUNK 512               // capacities are rounded up to it (a multiple of a mover item)
 #endif
-#define PIC_MOVER_THREADS 256
+#ifndef PIC_MOVER_THREADS
+#define PIC_MOVER_THREADS 128
+#endif
 #define PIC_FIX_SHIFT 40            // int64 deposit: 2^40 per unit deposit charge
 
 // Sticky device status bits (host maps them to PIC_ERR_*).
@@ -169,6 +171,19 @@ __device__ __forceinline__ void draw4(uint64_t seed, uint32_t pid, uint32_t step
 __device__ __forceinline__ uint32_t pack_cell(int i, int j) { return ((uint32_t)j << 16) | (uint32_t)i; }
 __device__ __forceinline__ int cell_i(uint32_t c) { return (int)(c & 0xFFFFu); }
 __device__ __forceinline__ int cell_j(uint32_t c) { return (int)(c >> 16); }
+
+// Reductions without a result on global memory.  Pointers that come out of the job and slot tables
+// are generic to the compiler, and a generic atomicAdd tests its address space on every call and
+// always returns the old value; these are plain red.global instructions.
+__device__ __forceinline__ void red_add(float* p, float v) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v));
+}
+__device__ __forceinline__ void red_add(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.global.add.u64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "l"(v));
+}
+__device__ __forceinline__ void red_add(int* p, int v) {
+  asm volatile("red.global.add.s32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(v));
+}
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 

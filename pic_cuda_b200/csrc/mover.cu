@@ -61,63 +61,54 @@ __device__ __forceinline__ void neutral_velocity(uint64_t seed, uint32_t pid, ui
   v[0] = sig * r0 * c; v[1] = sig * r0 * s; v[2] = sig * r1 * c2;
 }
 
-// Segmented sums towards each segment's first lane; maxlen (warp-uniform) bounds the segment
-// lengths, so only ceil(log2(maxlen)) shuffle levels run.
-template <typename T>
-__device__ __forceinline__ void seg_reduce4(T& a, T& b, T& c, T& d, int seg, int maxlen) {
-  const int lane = lane_id();
-  for (int o = 1; o < maxlen; o <<= 1) {
-    const T ta = __shfl_down_sync(0xffffffffu, a, o);
-    const T tb = __shfl_down_sync(0xffffffffu, b, o);
-    const T tc = __shfl_down_sync(0xffffffffu, c, o);
-    const T td = __shfl_down_sync(0xffffffffu, d, o);
-    const int ts = __shfl_down_sync(0xffffffffu, seg, o);
-    if (lane + o < 32 && ts == seg) { a += ta; b += tb; c += tc; d += td; }
-  }
-}
-
 }  // namespace
 
-// Particles per lane and per warp work item: lane l of a warp holds particles kPPL l ..
-// kPPL l + kPPL - 1 of a (32 kPPL)-particle item in registers, loaded with one vector load per
-// array (contiguous per warp and array).  Capacities are multiples of PIC_CHUNK, so every item
-// lies inside the arrays.  With the CTAs per SM below, measured on B200 (1025^2, 2e7
-// particles, ms per pass): 2 per lane at 4 CTAs per SM 0.441; 2 at 3 CTAs 0.466, at 5 CTAs
-// 0.476; 4 per lane at 3 CTAs 0.467, at 4 CTAs 0.510 (register spills).
+// Particles per lane and per warp work item: an item is kPPL / 2 blocks of 64 consecutive
+// particles, and lane l of a warp holds particles 2 l and 2 l + 1 of each block in registers, loaded
+// with one vector load per array and block (contiguous per warp).  The deposit sums block by block
+// (its FP32 rounding depends on the blocks, not on how many an item has).  Capacities are multiples
+// of PIC_CHUNK, so every item lies inside the arrays.  Small CTAs let the register file hold 28
+// warps of 72 registers.  Measured on B200, ms per pass at 1025^2 (2e7 particles, FP32 deposit) /
+// 4097^2 (2e8) / 4097^2 with the int64 deposit: one block, 128 threads x 7 CTAs per SM 0.341 / 3.22 /
+// 3.50; x 6 0.352 / 3.40 / 3.67; x 8 0.361 / 3.43 / 3.71; x 9 0.380 / 3.61 / 3.91; 256 x 4 0.356 /
+// 3.36 / 3.67; two blocks, 128 x 5 0.345 / 3.30 / 3.71; x 6 0.362 / 3.37 / 3.82.
 #ifndef PIC_MOVER_PPL
 #define PIC_MOVER_PPL 2
 #endif
 constexpr int kPPL = PIC_MOVER_PPL;
 constexpr int kItem = 32 * kPPL;
 
-// kPPL consecutive 4-byte values of one lane as one evict-first vector load / store.
-__device__ __forceinline__ void ld_lane(const float* p, float (&a)[4]) {
-  const float4 v = __ldcs(reinterpret_cast<const float4*>(p)); a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
+constexpr int kBlocks = kPPL / 2;
+// Particle k of a lane, relative to the item's first particle plus twice the lane.
+__device__ __forceinline__ constexpr int lane_at(int k) { return 64 * (k >> 1) + (k & 1); }
+
+// The kPPL 4-byte values of one lane, one evict-first 8-byte load / store per block (p: the lane's
+// first).
+__device__ __forceinline__ void ld_lane(const float* p, float (&a)[kPPL]) {
+#pragma unroll
+  for (int h = 0; h < kBlocks; ++h) {
+    const float2 v = __ldcs(reinterpret_cast<const float2*>(p + 64 * h));
+    a[2 * h] = v.x; a[2 * h + 1] = v.y;
+  }
 }
-__device__ __forceinline__ void ld_lane(const float* p, float (&a)[2]) {
-  const float2 v = __ldcs(reinterpret_cast<const float2*>(p)); a[0] = v.x; a[1] = v.y;
+__device__ __forceinline__ void ld_lane(const uint32_t* p, uint32_t (&a)[kPPL]) {
+#pragma unroll
+  for (int h = 0; h < kBlocks; ++h) {
+    const uint2 v = __ldcs(reinterpret_cast<const uint2*>(p + 64 * h));
+    a[2 * h] = v.x; a[2 * h + 1] = v.y;
+  }
 }
-__device__ __forceinline__ void ld_lane(const uint32_t* p, uint32_t (&a)[4]) {
-  const uint4 v = __ldcs(reinterpret_cast<const uint4*>(p)); a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
+__device__ __forceinline__ void st_lane(float* p, const float (&a)[kPPL]) {
+#pragma unroll
+  for (int h = 0; h < kBlocks; ++h) __stcs(reinterpret_cast<float2*>(p + 64 * h), make_float2(a[2 * h], a[2 * h + 1]));
 }
-__device__ __forceinline__ void ld_lane(const uint32_t* p, uint32_t (&a)[2]) {
-  const uint2 v = __ldcs(reinterpret_cast<const uint2*>(p)); a[0] = v.x; a[1] = v.y;
-}
-__device__ __forceinline__ void st_lane(float* p, const float (&a)[4]) {
-  __stcs(reinterpret_cast<float4*>(p), make_float4(a[0], a[1], a[2], a[3]));
-}
-__device__ __forceinline__ void st_lane(float* p, const float (&a)[2]) {
-  __stcs(reinterpret_cast<float2*>(p), make_float2(a[0], a[1]));
-}
-__device__ __forceinline__ void st_lane(uint32_t* p, const uint32_t (&a)[4]) {
-  __stcs(reinterpret_cast<uint4*>(p), make_uint4(a[0], a[1], a[2], a[3]));
-}
-__device__ __forceinline__ void st_lane(uint32_t* p, const uint32_t (&a)[2]) {
-  __stcs(reinterpret_cast<uint2*>(p), make_uint2(a[0], a[1]));
+__device__ __forceinline__ void st_lane(uint32_t* p, const uint32_t (&a)[kPPL]) {
+#pragma unroll
+  for (int h = 0; h < kBlocks; ++h) __stcs(reinterpret_cast<uint2*>(p + 64 * h), make_uint2(a[2 * h], a[2 * h + 1]));
 }
 constexpr int kWarps = PIC_MOVER_THREADS / 32;
 #ifndef PIC_MOVER_MIN_BLOCKS
-#define PIC_MOVER_MIN_BLOCKS 4
+#define PIC_MOVER_MIN_BLOCKS 7
 #endif
 
 // One real-or-null collision of a null-collision candidate (Vahedi & Surendra 1995): the
@@ -214,30 +205,6 @@ __device__ __forceinline__ void copy_words(void* dst, const void* src, int bytes
   for (int q = lane; q < bytes / 4; q += 32) d[q] = s[q];
 }
 
-// Segmented sum of the four corner weights of one run per lane over the warp (runs of equal
-// keys in lane order); the head lane of each segment adds the totals to rho.
-template <typename V>
-__device__ __forceinline__ void warp_runs_deposit(V* rho, int nx, uint32_t key, V v0, V v1, V v2, V v3) {
-  const int lane = lane_id();
-  const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
-  const bool head = (lane == 0) || (key != prev);
-  const unsigned heads = __ballot_sync(0xffffffffu, head);
-  const int seg = __popc(heads & (0xffffffffu >> (31 - lane)));
-  // longest segment: each lane measures its own from its head to the next head
-  const unsigned after = lane == 31 ? 0u : heads & (0xfffffffeu << lane);
-  const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-  const int next = after ? __ffs(after) - 1 : 32;
-  const int maxlen = (int)__reduce_max_sync(0xffffffffu, (unsigned)(next - first));
-  seg_reduce4(v0, v1, v2, v3, seg, maxlen);
-  if (head && key != PIC_CELL_OUT) {
-    V* r = rho + (size_t)cell_j(key) * nx + cell_i(key);
-    atomicAdd(r, v0);
-    atomicAdd(r + 1, v1);
-    atomicAdd(r + nx, v2);
-    atomicAdd(r + nx + 1, v3);
-  }
-}
-
 // CIC weights of one particle (updateDensity, kernels.cu:56-68) in deposit units: FP32, or
 // int64 fixed point whose four parts sum to the particle's quantised charge exactly.
 __device__ __forceinline__ void cic_f32(float q, float fx, float fy, float& a, float& b, float& c, float& d) {
@@ -252,30 +219,73 @@ __device__ __forceinline__ void cic_i64(long long qf, float fx, float fy, long l
   d = qf - a - b - c;
 }
 
-// Deposit of a lane's kPPL particles (keys in lane order): runs of equal keys inside the lane
-// are summed in registers; every finished run but the lane's last goes to rho directly, and
-// the last runs of all lanes go through one warp-segmented reduction.  Called by all lanes.
-template <typename V, typename W>
-__device__ __forceinline__ void lane_deposit(V* rho, int nx, const uint32_t key[kPPL], const float fx[kPPL],
-                                             const float fy[kPPL], W weights) {
-  V a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-  uint32_t rk = key[0];
-  if (rk != PIC_CELL_OUT) weights(fx[0], fy[0], a0, a1, a2, a3);
+// Deposit of H blocks of 64 particles, two per lane and block (keys in lane order).  Per block: equal
+// keys of a lane's pair are summed in registers (of two different ones the first goes to rho at
+// once), then the lanes' runs of equal keys are summed over the warp (lane order) and the first lane
+// of each adds the totals to rho.  The blocks' reductions run together.  Called by all lanes.
+template <int H, typename V, typename W>
+__device__ __forceinline__ void lane_deposit(V* rho, int nx, const uint32_t* key, const float* fx, const float* fy,
+                                             W weights) {
+  const int lane = lane_id();
+  V v[H][4];
+  uint32_t rk[H];
+  int end[H];
+  bool head[H];
+  int longest = 0;
 #pragma unroll
-  for (int k = 1; k < kPPL; ++k) {
-    V b0 = 0, b1 = 0, b2 = 0, b3 = 0;
-    if (key[k] != PIC_CELL_OUT) weights(fx[k], fy[k], b0, b1, b2, b3);
-    if (key[k] == rk) {
-      a0 += b0; a1 += b1; a2 += b2; a3 += b3;
+  for (int h = 0; h < H; ++h) {
+    V b[4] = {0, 0, 0, 0};
+    v[h][0] = v[h][1] = v[h][2] = v[h][3] = 0;
+    rk[h] = key[2 * h];
+    if (rk[h] != PIC_CELL_OUT) weights(fx[2 * h], fy[2 * h], v[h][0], v[h][1], v[h][2], v[h][3]);
+    if (key[2 * h + 1] != PIC_CELL_OUT) weights(fx[2 * h + 1], fy[2 * h + 1], b[0], b[1], b[2], b[3]);
+    if (key[2 * h + 1] == rk[h]) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[h][u] += b[u];
     } else {
-      if (rk != PIC_CELL_OUT) {
-        V* r = rho + (size_t)cell_j(rk) * nx + cell_i(rk);
-        atomicAdd(r, a0); atomicAdd(r + 1, a1); atomicAdd(r + nx, a2); atomicAdd(r + nx + 1, a3);
+      if (rk[h] != PIC_CELL_OUT) {
+        V* r = rho + (size_t)cell_j(rk[h]) * nx + cell_i(rk[h]);
+        red_add(r, v[h][0]); red_add(r + 1, v[h][1]); red_add(r + nx, v[h][2]); red_add(r + nx + 1, v[h][3]);
       }
-      rk = key[k]; a0 = b0; a1 = b1; a2 = b2; a3 = b3;
+      rk[h] = key[2 * h + 1];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[h][u] = b[u];
     }
   }
-  warp_runs_deposit(rho, nx, rk, a0, a1, a2, a3);
+#pragma unroll
+  for (int h = 0; h < H; ++h) {
+    const uint32_t prev = __shfl_up_sync(0xffffffffu, rk[h], 1);
+    head[h] = (lane == 0) || (rk[h] != prev);
+    const unsigned heads = __ballot_sync(0xffffffffu, head[h]);
+    // the lane after this lane's segment, and the segment's length from its head
+    const unsigned after = lane == 31 ? 0u : heads & (0xfffffffeu << lane);
+    const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+    end[h] = after ? __ffs(after) - 1 : 32;
+    longest = max(longest, end[h] - first);
+  }
+  longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)longest);
+  // only as many shuffle levels as the longest segment needs
+  for (int o = 1; o < longest; o <<= 1) {
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      V t[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) t[u] = __shfl_down_sync(0xffffffffu, v[h][u], o);
+      if (lane + o < end[h]) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[h][u] += t[u];
+      }
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < H; ++h)
+    if (head[h] && rk[h] != PIC_CELL_OUT) {
+      V* r = rho + (size_t)cell_j(rk[h]) * nx + cell_i(rk[h]);
+      red_add(r, v[h][0]);
+      red_add(r + 1, v[h][1]);
+      red_add(r + nx, v[h][2]);
+      red_add(r + nx + 1, v[h][3]);
+    }
 }
 
 // Deferred collision candidates of a warp: cell fx fy vx vy vz pid index, up to one round of
@@ -317,10 +327,11 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
   int qn = 0;                                                      // queued candidates (warp-uniform)
   if (lane < 8) pc[lane] = 0u;
   __syncwarp();
-  int cur = -1;
+  int cur = -1, cur_first = 0, cur_end = 0;   // the warp's slot, its first item and the one after its last
   double ke = 0.0;
   bool do_kick = false, do_mcc = false, do_drift = false, do_walls = false, do_dep = false, want_ke = false;
   uint32_t mcc_step = 0;
+  uint32_t cand_below = 0;   // draws m with u01 = (2 m + 1) 2^-24 < pnull: exactly those m < cand_below
   int n = 0;
   // One round over the first cnt queued candidates (one per lane): collide (Philox stream
   // (seed, pid, step) as for the candidate test), drift, absorb, deposit, store at the
@@ -380,10 +391,12 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
   };
   const int nwarps = gridDim.x * kWarps;
   for (int item = blockIdx.x * kWarps + warp; item < total; item += nwarps) {
-    int s = cur < 0 ? 0 : cur;
-    while (s < nslots - 1 && item_prefix[s + 1] <= item) ++s;
-    if (s != cur) {
+    if (item >= cur_end) {
+      int s = cur < 0 ? 0 : cur;
+      while (s < nslots - 1 && item_prefix[s + 1] <= item) ++s;
       flush();
+      cur_first = item_prefix[s];
+      cur_end = item_prefix[s + 1];
       copy_words(&tab[warp].S, slots + s, sizeof(SlotDev), lane);
       __syncwarp();
       copy_words(&tab[warp].J, jobs + S.job, sizeof(JobDev), lane);
@@ -400,8 +413,10 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
       want_ke = do_kick || do_mcc;
       mcc_step = gated ? (uint32_t)(T0.step - 1) : explicit_step;
       n = counts[s];
+      cand_below = (uint32_t)ceil((fmin((double)S.pnull, 1.0) * 16777216.0 - 1.0) * 0.5);
     }
-    const int i0 = (item - item_prefix[s]) * kItem + kPPL * lane;
+    const int s = cur;
+    const int i0 = (item - cur_first) * kItem + 2 * lane;
     // ---- loads
     uint32_t c[kPPL], pid[kPPL];
     float fx[kPPL], fy[kPPL], vx[kPPL], vy[kPPL], vz[kPPL];
@@ -421,7 +436,7 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
     }
     bool valid[kPPL];
 #pragma unroll
-    for (int k = 0; k < kPPL; ++k) valid[k] = i0 + k < n;
+    for (int k = 0; k < kPPL; ++k) valid[k] = i0 + lane_at(k) < n;
     // ---- pass A: kick and collisions
     if (do_kick) {
       const float2* __restrict__ ef = J.efield;
@@ -459,24 +474,41 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
             }
           }
       } else {
+        // candidate with probability nu_max dt; a candidate's collision is real when
+        // u1 nu_max < n sigma_T(E) v (the process is chosen in the queue round, with the
+        // same draw).  Null candidates stay in the item like every other particle.
         bool cand[kPPL];
+        uint32_t x1[kPPL];
         unsigned m[kPPL];
         int before[kPPL];
         int ncand = 0;
 #pragma unroll
         for (int k = 0; k < kPPL; ++k) {
-          // candidate with probability nu_max dt; a candidate's collision is real when
-          // u1 nu_max < n sigma_T(E) v (the process is chosen in the queue round, with the
-          // same draw).  Null candidates stay in the item like every other particle.
-          cand[k] = false;
-          if (valid[k]) {
-            float u[4];
-            draw4(J.seed, pid[k], mcc_step, 0u, u);
-            if (u[0] < S.pnull) {
-              const float v2 = vx[k] * vx[k] + vy[k] * vy[k] + vz[k] * vz[k];
-              cand[k] = u[1] * S.numax < J.gas_density * xs_lookup(S.total, S.half_m_over_e * v2) * sqrtf(v2);
-            }
-          }
+          uint32_t x[4] = {pid[k], mcc_step, 0u, 0u};
+          philox4x32_10(x, (uint32_t)J.seed, (uint32_t)(J.seed >> 32));
+          x1[k] = x[1];
+          cand[k] = valid[k] && (x[0] >> 9) < cand_below;
+        }
+        // The cross-section lookup is a chain of dependent loads that the whole warp waits for
+        // whenever one lane needs it, so each pass of this loop takes one candidate of every lane
+        // that has any left: one pass where each lane has at most one.
+        unsigned left = 0;
+#pragma unroll
+        for (int k = 0; k < kPPL; ++k) left |= cand[k] ? 1u << k : 0u;
+        while (left) {
+          const int k = __ffs(left) - 1;
+          left &= left - 1u;
+          float v2 = 0.f, u1 = 0.f;
+#pragma unroll
+          for (int q = 0; q < kPPL; ++q)
+            if (q == k) { v2 = vx[q] * vx[q] + vy[q] * vy[q] + vz[q] * vz[q]; u1 = u01(x1[q]); }
+          const bool real = u1 * S.numax < J.gas_density * xs_lookup(S.total, S.half_m_over_e * v2) * sqrtf(v2);
+#pragma unroll
+          for (int q = 0; q < kPPL; ++q)
+            if (q == k) cand[q] = real;
+        }
+#pragma unroll
+        for (int k = 0; k < kPPL; ++k) {
           m[k] = __ballot_sync(0xffffffffu, cand[k]);
           before[k] = ncand;
           ncand += __popc(m[k]);
@@ -494,7 +526,7 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
             cq[1 * kQueue + q] = __float_as_uint(fx[k]); cq[2 * kQueue + q] = __float_as_uint(fy[k]);
             cq[3 * kQueue + q] = __float_as_uint(vx[k]); cq[4 * kQueue + q] = __float_as_uint(vy[k]);
             cq[5 * kQueue + q] = __float_as_uint(vz[k]); cq[6 * kQueue + q] = pid[k];
-            cq[7 * kQueue + q] = (uint32_t)(i0 + k);
+            cq[7 * kQueue + q] = (uint32_t)(i0 + lane_at(k));
             valid[k] = false;   // the queue round finishes this particle
           }
         qn += ncand;
@@ -515,10 +547,30 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
     for (int k = 0; k < kPPL; ++k) {
       absorbed[k] = false;
       key[k] = valid[k] ? c[k] : PIC_CELL_OUT;
-      if (do_drift && valid[k]) {
-        const Drifted d = drift_particle(J, S, c[k], fx[k], fy[k], vx[k], vy[k], do_walls);
-        absorbed[k] = d.absorbed; c[k] = d.cell; fx[k] = d.fx; fy[k] = d.fy;
-        key[k] = d.absorbed ? PIC_CELL_OUT : d.cell;
+    }
+    if (do_drift) {
+      // no particle of the warp leaves its cell (ions, nearly always): the drifted offsets are the
+      // new ones and nothing is absorbed, without the cell arithmetic
+      bool stay = !(do_walls && (J.wall_mode & 2));
+      float ax[kPPL], ay[kPPL];
+#pragma unroll
+      for (int k = 0; k < kPPL; ++k) {
+        ax[k] = fx[k] + vx[k] * S.dtdx;
+        ay[k] = fy[k] + vy[k] * S.dtdy;
+        stay = stay && (!valid[k] || (c[k] != PIC_CELL_OUT && ax[k] >= 0.f && ax[k] < 1.f && ay[k] >= 0.f && ay[k] < 1.f));
+      }
+      if (__all_sync(0xffffffffu, stay)) {
+#pragma unroll
+        for (int k = 0; k < kPPL; ++k)
+          if (valid[k]) { fx[k] = ax[k]; fy[k] = ay[k]; }
+      } else {
+#pragma unroll
+        for (int k = 0; k < kPPL; ++k)
+          if (valid[k]) {
+            const Drifted d = drift_particle(J, S, c[k], fx[k], fy[k], vx[k], vy[k], do_walls);
+            absorbed[k] = d.absorbed; c[k] = d.cell; fx[k] = d.fx; fy[k] = d.fy;
+            key[k] = d.absorbed ? PIC_CELL_OUT : d.cell;
+          }
       }
     }
     if (do_walls) {
@@ -536,25 +588,30 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
         base = __shfl_sync(0xffffffffu, base, 0);
 #pragma unroll
         for (int k = 0; k < kPPL; ++k)
-          if (valid[k] && absorbed[k]) S.hits[base + hb[k] + __popc(hm[k] & ((1u << lane) - 1u))] = i0 + k;
+          if (valid[k] && absorbed[k]) S.hits[base + hb[k] + __popc(hm[k] & ((1u << lane) - 1u))] = i0 + lane_at(k);
       }
     }
     if (do_dep) {
       if (J.deposit_mode == 0) {
         const float q = S.qdep;
-        lane_deposit<float>(J.rho_f, J.nx, key, fx, fy,
-                            [q](float x, float y, float& a, float& b, float& cc, float& d) { cic_f32(q, x, y, a, b, cc, d); });
+        lane_deposit<kBlocks, float>(J.rho_f, J.nx, key, fx, fy,
+                                     [q](float x, float y, float& a, float& b, float& cc, float& d) {
+                                       cic_f32(q, x, y, a, b, cc, d);
+                                     });
       } else {
+        // block by block: the 64-bit sums of several blocks do not fit the registers
         const long long qf = S.qfix;
-        lane_deposit<unsigned long long>(
-            reinterpret_cast<unsigned long long*>(J.rho_i), J.nx, key, fx, fy,
-            [qf](float x, float y, unsigned long long& a, unsigned long long& b, unsigned long long& cc,
-                 unsigned long long& d) {
-              long long a_, b_, c_, d_;
-              cic_i64(qf, x, y, a_, b_, c_, d_);
-              a = (unsigned long long)a_; b = (unsigned long long)b_; cc = (unsigned long long)c_;
-              d = (unsigned long long)d_;
-            });
+#pragma unroll
+        for (int h = 0; h < kBlocks; ++h)
+          lane_deposit<1, unsigned long long>(
+              reinterpret_cast<unsigned long long*>(J.rho_i), J.nx, key + 2 * h, fx + 2 * h, fy + 2 * h,
+              [qf](float x, float y, unsigned long long& a, unsigned long long& b, unsigned long long& cc,
+                   unsigned long long& d) {
+                long long a_, b_, c_, d_;
+                cic_i64(qf, x, y, a_, b_, c_, d_);
+                a = (unsigned long long)a_; b = (unsigned long long)b_; cc = (unsigned long long)c_;
+                d = (unsigned long long)d_;
+              });
       }
     }
     // ---- stores

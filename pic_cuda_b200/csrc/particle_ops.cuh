@@ -75,18 +75,18 @@ __device__ __forceinline__ void deposit_one(const JobDev& J, const SlotDev& S, u
   const size_t a = (size_t)j * J.nx + i;
   const float w00 = (1.f - fx) * (1.f - fy), w10 = fx * (1.f - fy), w01 = (1.f - fx) * fy, w11 = fx * fy;
   if (J.deposit_mode == 0) {
-    atomicAdd(J.rho_f + a, S.qdep * w00);
-    atomicAdd(J.rho_f + a + 1, S.qdep * w10);
-    atomicAdd(J.rho_f + a + J.nx, S.qdep * w01);
-    atomicAdd(J.rho_f + a + J.nx + 1, S.qdep * w11);
+    red_add(J.rho_f + a, S.qdep * w00);
+    red_add(J.rho_f + a + 1, S.qdep * w10);
+    red_add(J.rho_f + a + J.nx, S.qdep * w01);
+    red_add(J.rho_f + a + J.nx + 1, S.qdep * w11);
   } else {
     const double Q = (double)S.qfix;
     const long long v0 = __double2ll_rn((double)w00 * Q), v1 = __double2ll_rn((double)w10 * Q);
     const long long v2 = __double2ll_rn((double)w01 * Q), v3 = S.qfix - v0 - v1 - v2;
     unsigned long long* rho = (unsigned long long*)J.rho_i;
-    atomicAdd(rho + a, (unsigned long long)v0);
-    atomicAdd(rho + a + 1, (unsigned long long)v1);
-    atomicAdd(rho + a + J.nx, (unsigned long long)v2);
-    atomicAdd(rho + a + J.nx + 1, (unsigned long long)v3);
+    red_add(rho + a, (unsigned long long)v0);
+    red_add(rho + a + 1, (unsigned long long)v1);
+    red_add(rho + a + J.nx, (unsigned long long)v2);
+    red_add(rho + a + J.nx + 1, (unsigned long long)v3);
   }
 }

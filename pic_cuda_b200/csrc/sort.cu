@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(256) sort_hist(const JobDev* jobs, const SlotD
     for (int r = 0; r < kSortRounds; ++r) {
       int first, last;
       run_segment(key[r], first, last);
-      if (lane == last && key[r] != kNoKey) atomicAdd(cnt + key[r], last - first + 1);
+      if (lane == last && key[r] != kNoKey) red_add(cnt + key[r], last - first + 1);
       if (count_descents) {
         uint32_t prev = __shfl_up_sync(0xffffffffu, key[r], 1);
         const uint32_t wrap = r > 0 ? __shfl_sync(0xffffffffu, key[r > 0 ? r - 1 : 0], 31) : kNoKey;
