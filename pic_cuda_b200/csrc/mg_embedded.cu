@@ -30,6 +30,8 @@
 //   emb_smooth_kernel<NU, PRO>  the same tile scheme with a halo of 2 NU for the
 //       post-smoothing: the coarse correction is prolongated while staging (PRO).  Tiles read
 //       halos that neighbouring CTAs own, so results go to the level's other phi buffer.
+//   Levels with enough nodes (strip_args) run the same smoothing as pipelines of rows in registers
+//       (emb_strip_kernel, emb_strips.cuh), with the same bits.
 //   emb_coarse_kernel  every level from the first one with at most 65 x 65 nodes down, in one
 //       CTA's shared memory (one launch for the whole lower V-cycle).
 //   emb_norm_kernel / emb_norm_final_kernel  ||r||^2 and ||rhs||^2 over the FLUID nodes in a
@@ -43,6 +45,7 @@
 #include <mutex>
 #include <vector>
 #include "common.cuh"
+#include "emb_strips.cuh"
 #include "kernels.h"
 
 int pic_fail(int code, const char* msg);
@@ -476,9 +479,47 @@ int coarse_smem_bytes(const EmbLevels& P, int l0, int offs[PIC_MAX_LEVELS]) {
   return off;
 }
 
+// Arguments of the strip kernels (emb_strips.cuh) for nu sweeps of a level (down: with the
+// restriction); rows = 0 where the tile kernels take it.  An item is one warp with FP64 chains to hide, so
+// a level needs about 14 of them per SM; the largest row count that still gives as many wastes
+// least on the rows a strip recomputes, up to 36 (more leave the last wave empty).  Measured on
+// B200, V-cycle at 4097^2 with at most 36 / 48 / 60 rows: 532 / 539 / 536 us at 14 items per SM, 532 /
+// 554 / 562 at 10, 589 / 591 / 592 at 18; tiles alone 772.  At 2049^2 238 against 273 us; at 1025^2 the
+// strips (10 per SM) would lose, 138 against 136.
+embs::Args strip_args(const EmbLevels& P, int l, int nu, bool down, const double* in, double* out) {
+  constexpr int kItemsPerSm = 14, kMaxRows = 36;
+  embs::Args A{};
+  const int nx = P.nx[l], ny = P.ny[l];
+  if (nu > embs::kMaxNu || (int64_t)nx * ny >= 1 << 30) return A;   // 32-bit node positions
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return A;
+  }
+  A.phi = in; A.out = out; A.rhs = P.rhs[l]; A.mask = P.mask[l]; A.bc = P.bc[l];
+  A.nx = nx; A.ny = ny;
+  A.h2 = P.h * P.h * std::ldexp(1.0, 2 * l);
+  A.strips_x = embs::strips(nu, down, nx);
+  for (int rows = embs::rows_fit(nu, down, kMaxRows); rows > 0; rows = embs::rows_fit(nu, down, rows - 1)) {
+    const int64_t items = (int64_t)A.strips_x * ((ny + rows - 1) / rows);
+    if (items >= (int64_t)kItemsPerSm * sms) { A.rows = rows; A.items = (int)items; break; }
+  }
+  return A;
+}
+
 template <int NU, bool PRO>
 void launch_smooth(const EmbLevels& P, int l, const double* in, double* out, const double* coarse, bool bilinear,
                    cudaStream_t s) {
+  if constexpr (NU <= embs::kMaxNu) {
+    embs::Args A = strip_args(P, l, NU, false, in, out);
+    if (A.rows) {
+      A.coarse = coarse;
+      A.bilinear = bilinear ? 1 : 0;
+      if (PRO) { A.nxc = P.nx[l + 1]; A.nyc = P.ny[l + 1]; }
+      embs::emb_strip_kernel<NU, false, PRO><<<(A.items + embs::kWarps - 1) / embs::kWarps, 32 * embs::kWarps, 0, s>>>(A);
+      return;
+    }
+  }
   const dim3 grid((P.nx[l] + kTile - 1) / kTile, (P.ny[l] + kTile - 1) / kTile);
   const double h2 = P.h * P.h * std::ldexp(1.0, 2 * l);
   emb_smooth_kernel<NU, PRO><<<grid, kSmoothThreads, 0, s>>>(in, out, P.rhs[l], P.mask[l], P.bc[l], coarse, P.nx[l],
@@ -504,6 +545,16 @@ void smooth_chunk(const EmbLevels& P, int l, int nu, bool pro, const double* in,
 
 template <int NU>
 void launch_down(const EmbLevels& P, int l, const double* in, double* out, int any, cudaStream_t s) {
+  if constexpr (NU <= embs::kMaxNu) {
+    embs::Args A = strip_args(P, l, NU, true, in, out);
+    if (A.rows) {
+      A.nxc = P.nx[l + 1]; A.nyc = P.ny[l + 1];
+      A.rhs_c = P.rhs[l + 1]; A.mask_c = P.mask[l + 1]; A.phi_c = P.phi[l + 1];
+      A.any = any;
+      embs::emb_strip_kernel<NU, true, false><<<(A.items + embs::kWarps - 1) / embs::kWarps, 32 * embs::kWarps, 0, s>>>(A);
+      return;
+    }
+  }
   const dim3 grid((P.nx[l] + kTile - 1) / kTile, (P.ny[l] + kTile - 1) / kTile);
   const double h2 = P.h * P.h * std::ldexp(1.0, 2 * l);
   emb_down_kernel<NU><<<grid, kSmoothThreads, 0, s>>>(in, out, P.rhs[l], P.mask[l], P.bc[l], P.nx[l], P.ny[l], h2,

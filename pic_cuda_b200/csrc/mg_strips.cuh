@@ -278,7 +278,7 @@ struct UpArgs {
 // copy of theirs can be wider than one value: lane k copies columns k and k + 32, which keeps each
 // copy contiguous over the warp, and the lanes read their pairs after a warp barrier.
 template <int MODE>
-struct UpStep {
+struct __align__(16) UpStep {
   float2 e[32], f[32], c[32];
   double phi[MODE ? 64 : 1], rho[MODE ? 64 : 1];
 };
