@@ -71,6 +71,7 @@ struct JobHost {
   int64_t bytes = 0;
   int64_t steps = 0;
   bool pending = false;
+  bool loaded = false;     // particles were loaded since the job's last sort (in no cell order)
   // JobState::total_charge holds the sum of the present rho: the level-0 residual kernel
   // of every field solve computes it; entry points that change rho otherwise clear this
   bool charge_fresh = false;
@@ -698,12 +699,14 @@ int check_job(pic_engine* E, int job) {
 template <typename Due>
 int sort_jobs(pic_engine* E, const EngineLaunch& L, Due due, cudaStream_t s, bool* launched) {
   std::vector<uint8_t> mask(L.nslots, 0);
-  bool any = false;
+  bool any = false, loaded = false;
   int max_cells = 0;
   int64_t max_p = 0;
   for (int j = 0; j < E->njobs_hw; ++j) {
     JobHost& J = E->jobs[j];
     if (!J.alive || J.cfg.sort_every <= 0 || !due(J)) continue;
+    loaded |= J.loaded;
+    J.loaded = false;
     for (int k = 0; k < J.cfg.n_species; ++k) {
       mask[j * kSlotsPerJob + k] = 1;
       max_p = std::max<int64_t>(max_p, J.cfg.species[k].capacity);
@@ -715,7 +718,7 @@ int sort_jobs(pic_engine* E, const EngineLaunch& L, Due due, cudaStream_t s, boo
   if (!any) return PIC_OK;
   CK(cudaMemcpyAsync(E->d_mask, mask.data(), mask.size(), cudaMemcpyHostToDevice, s));
   phase_mark(E, 0, true, s);
-  E->launches += launch_sort(L, E->d_mask, max_cells, (int)std::min<int64_t>(max_p, 1 << 30), true, s);
+  E->launches += launch_sort(L, E->d_mask, max_cells, (int)std::min<int64_t>(max_p, 1 << 30), true, loaded, s);
   phase_mark(E, 0, false, s);
   return PIC_OK;
 }
@@ -811,7 +814,7 @@ int build_step_graph(pic_engine* E, bool with_sort, cudaGraphExec_t* out, int64_
       max_cells = std::max(max_cells, J.dev.ncx * J.dev.ncy);
     }
     n += launch_sort_mask(L, E->d_mask, 1, E->side_stream);
-    n += launch_sort(L, E->d_mask, max_cells, (int)std::min<int64_t>(max_p, 1 << 30), true, E->side_stream);
+    n += launch_sort(L, E->d_mask, max_cells, (int)std::min<int64_t>(max_p, 1 << 30), true, false, E->side_stream);
   }
   if (err == cudaSuccess) err = cudaEventRecord(E->ev_join, E->side_stream);
   n += launch_mg_init(L, E->mg_all.L, s);
@@ -1363,6 +1366,7 @@ int pic_job_load_species(pic_engine* E, int job, int species, int64_t n, const d
   const SlotDev* sd = E->d_slots + job * kSlotsPerJob + species;
   launch_load_species(sd, nullptr, n, dx_, dy_, dvx, dvy, dvz, dpid, hs.next_pid, 1.0 / dxv, 1.0 / dyv, J.dev.ncx,
                       J.dev.ncy, s);
+  J.loaded = true;
   const int ni = (int)n;
   CK(cudaMemcpyAsync(E->d_counts + job * kSlotsPerJob + species, &ni, sizeof(int), cudaMemcpyHostToDevice, s));
   if (dpid) {
@@ -1666,7 +1670,8 @@ int pic_job_sort(pic_engine* E, int job, void* stream) {
   int64_t maxp = 0;
   for (int k = 0; k < J.cfg.n_species; ++k) maxp = std::max<int64_t>(maxp, J.cfg.species[k].capacity);
   EngineLaunch L = make_launch(E, nullptr);
-  launch_sort(L, E->d_mask, J.dev.ncx * J.dev.ncy, (int)std::min<int64_t>(maxp, 1 << 30), false, s);
+  launch_sort(L, E->d_mask, J.dev.ncx * J.dev.ncy, (int)std::min<int64_t>(maxp, 1 << 30), false, J.loaded, s);
+  J.loaded = false;
   CK(cudaStreamSynchronize(s));
   CK(cudaGetLastError());
   return PIC_OK;

@@ -48,8 +48,9 @@ int launch_ionize(const EngineLaunch& L, bool drift_and_deposit, cudaStream_t s)
 // Counting sort of the slots in sort_mask; by_disorder: the histogram pass also counts the
 // particles that follow a particle of a later cell (aux[4 s + 3]), and slots where they are
 // fewer than 1/32 of the particles are left as they are.
+// random_order: the particles were loaded since the last sort, so large slots take the band pass.
 int launch_sort(const EngineLaunch& L, uint8_t* sort_mask, int max_cells, int max_particles, bool by_disorder,
-                cudaStream_t s);
+                bool random_order, cudaStream_t s);
 int launch_step_begin(JobState* st, const JobDev* jobs, int njobs, const uint8_t* job_mask, cudaStream_t s);
 int launch_ke_reset_pending(JobState* st, int njobs, cudaStream_t s);
 int launch_step_end(JobState* st, int njobs, const uint8_t* job_mask, int set_pending, int advance, cudaStream_t s);

@@ -16,6 +16,9 @@
 namespace {
 
 constexpr int kTile = 2048;     // cells per scan tile (256 threads x 8)
+// Freshly loaded slots of at least this many particles take the band pass (below, a slot's arrays sit
+// in L2 anyway: 1.3 M particles 0.224 ms without it, 0.229 with; 2.6 M 0.456 and 0.435).
+constexpr int kBandMinParticles = 2000000;
 
 __device__ __forceinline__ uint32_t dense_key(uint32_t c, int ncx, uint32_t ncells) {
   return c == PIC_CELL_OUT ? ncells : (uint32_t)cell_j(c) * (uint32_t)ncx + (uint32_t)cell_i(c);
@@ -52,6 +55,7 @@ __device__ __forceinline__ void run_segment(uint32_t key, int& first, int& last)
 // warp keeps kSortRounds coalesced requests per array in flight.
 constexpr int kSortRounds = 4;
 constexpr int kSortItem = 32 * kSortRounds;
+constexpr int kScatterCtas = 2;   // of the scatter, per SM: all resident at once
 
 // Histogram of cell keys, one atomic per warp segment of equal keys.  With count_descents, also
 // the particles whose key is below their predecessor's (within a warp iteration's 4 x 32), one
@@ -151,12 +155,14 @@ __global__ void __launch_bounds__(256) sort_tile_sums(const JobDev* jobs, const 
   }
 }
 
-__global__ void __launch_bounds__(256) sort_scan_parts(const JobDev* jobs, const SlotDev* slots, const uint8_t* mask) {
+__global__ void __launch_bounds__(256) sort_scan_parts(const JobDev* jobs, const SlotDev* slots, const uint8_t* mask,
+                                                      int* aux) {
   const int s = blockIdx.x;
   if (!mask[s]) return;
   const SlotDev& S = slots[s];
   const JobDev& J = jobs[S.job];
   const int ntiles = (J.ncx * J.ncy + 1 + kTile - 1) / kTile;
+  if (threadIdx.x == 0) aux[4 * s + 3] = 0;   // the scatter's tickets
   int carry = 0;
   for (int b = 0; b < ntiles; b += kTile) {
     int v[8];
@@ -201,7 +207,16 @@ __global__ void __launch_bounds__(256) sort_apply(const JobDev* jobs, const Slot
 // segment of equal keys returns the segment's first position.  Every field of the warp's
 // kSortRounds x 32 particles is loaded before the atomics, so loads and atomics overlap; the
 // stores of a round are consecutive across lanes where the order was kept since the last sort.
-__global__ void sort_scatter(const JobDev* jobs, const SlotDev* slots, const int* counts, const uint8_t* mask) {
+//
+// Warps take their items from a ticket counter (aux[4 s + 3]), in order.  The destinations of a stretch
+// of the slot spread over the rows its particles reached; they are filled by later stretches too, and
+// only while all warps stay within a few rows of one another do the part-filled sectors wait for that
+// in L2.  With a grid-stride loop the warps drifted apart over the pass (and with more CTAs than fit, the
+// second wave went over the slot again): twice the traffic.  Two CTAs per SM keep the stretch in
+// flight small.  Measured on B200, a steady-state sort of the electrons (1e7 at 1025^2 / 2.5e7 at 2049^2 /
+// 1e8 at 4097^2): grid stride 0.56 / 1.32 / 6.7 ms; tickets, 2 CTAs per SM 0.42 / 1.04 / 3.94; 1 CTA 0.48 /
+// 1.15 / 4.65; 3 CTAs 0.46 / 1.05 / 4.00; four items a ticket, 2 CTAs 0.50 / 1.12 / 4.22.
+__global__ void __launch_bounds__(256, kScatterCtas) sort_scatter(const JobDev* jobs, const SlotDev* slots, const int* counts, const uint8_t* mask, int* aux) {
   const int s = blockIdx.y;
   if (!mask[s]) return;
   const SlotDev& S = slots[s];
@@ -226,7 +241,13 @@ __global__ void sort_scatter(const JobDev* jobs, const SlotDev* slots, const int
   int* const cnt = S.cell_count;
   const int lane = lane_id();
   const int nitems = (n + kSortItem - 1) / kSortItem;
-  for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < nitems; it += (gridDim.x * blockDim.x) >> 5) {
+  int* const ticket = aux + 4 * s + 3;
+  auto take = [&]() { return lane == 0 ? atomicAdd(ticket, 1) : 0; };
+  int taken = take();
+  for (;;) {
+    const int it = __shfl_sync(0xffffffffu, taken, 0);
+    if (it >= nitems) break;
+    taken = take();   // the next item's ticket arrives behind this one's loads
     uint32_t c[kSortRounds], pd[kSortRounds], key[kSortRounds];
     float a[kSortRounds], b[kSortRounds], u[kSortRounds], v[kSortRounds], w[kSortRounds];
 #pragma unroll
@@ -256,6 +277,125 @@ __global__ void sort_scatter(const JobDev* jobs, const SlotDev* slots, const int
   }
 }
 
+// ---- band pass, for particles in arbitrary order (freshly loaded)
+// The scatter above writes every 4-byte field of a randomly placed particle to a random place of the
+// slot: a sector of its own, seldom completed while it is in L2.  Before it, such a slot is grouped
+// into kBands bands of cell rows, each of which (16 M / 128 cells' particles at most) stays in L2 while
+// the scatter fills it.  A CTA ranks a chunk of kBandChunk particles by band in shared memory and then
+// moves one field at a time through it, so that a band's particles of the chunk (16 of a random order)
+// leave as one run; the bands' first places come from the scanned cell counts.  Measured on B200, first
+// sort of two random slots (histogram, scans and both passes), without / with the pass and with the
+// scatter's tickets: 1e7 each at 1025^2 5.1 / 1.75 / 1.52 ms, 2.5e7 at 2049^2 15.9 / 7.7 / 3.81, 1e8 at 4097^2
+// 71.8 / 67.7 / 18.1; 256 bands 1.56 / 3.90 / 17.6 with both.
+constexpr int kBands = 128;
+constexpr int kBandThreads = 256;
+constexpr int kBandPer = 8;                               // particles per thread and chunk
+constexpr int kBandChunk = kBandThreads * kBandPer;
+constexpr int kBandSums = (kBands + 1 + 31) / 32;         // bands per lane of the scan
+
+__device__ __forceinline__ int bands_of(const JobDev& J) { return min(kBands, J.ncy); }
+__device__ __forceinline__ bool banded_slot(const JobDev& J, int n) {
+  return n >= kBandMinParticles && J.ncx * J.ncy >= 4 * kBands;
+}
+// band of a cell: rows split into nb bands; particles outside the grid go last
+__device__ __forceinline__ int band_of(uint32_t c, int ncy, int nb) {
+  return c == PIC_CELL_OUT ? nb : (int)(((uint32_t)cell_j(c) * (uint32_t)nb) / (uint32_t)ncy);
+}
+
+// The bands' first places (the compaction's list array holds them between compactions).
+__global__ void sort_band_init(const JobDev* jobs, const SlotDev* slots, const int* counts, const uint8_t* mask) {
+  const int s = blockIdx.x;
+  if (!mask[s]) return;
+  const SlotDev& S = slots[s];
+  const JobDev& J = jobs[S.job];
+  if (!banded_slot(J, counts[s])) return;
+  const int nb = bands_of(J);
+  for (int b = threadIdx.x; b <= nb; b += blockDim.x) {
+    const int row = b == nb ? J.ncy : (b * J.ncy + nb - 1) / nb;   // the band's first row
+    S.scratch2[b] = S.cell_count[row * J.ncx];
+  }
+}
+
+__global__ void __launch_bounds__(kBandThreads) sort_band_scatter(const JobDev* jobs, const SlotDev* slots,
+                                                                  const int* counts, const uint8_t* mask) {
+  const int s = blockIdx.y;
+  if (!mask[s]) return;
+  const SlotDev& S = slots[s];
+  const JobDev& J = jobs[S.job];
+  const int n = counts[s];
+  if (!banded_slot(J, n)) return;
+  __shared__ int h[kBands + 1], off[32 * kBandSums], base[kBands + 1];
+  __shared__ int place[kBandChunk];
+  __shared__ uint32_t stage[2][kBandChunk];
+  const int nb = bands_of(J), ncy = J.ncy, t = threadIdx.x;
+  const uint32_t* const src[7] = {S.cell, reinterpret_cast<const uint32_t*>(S.fx), reinterpret_cast<const uint32_t*>(S.fy),
+                                  reinterpret_cast<const uint32_t*>(S.vx), reinterpret_cast<const uint32_t*>(S.vy),
+                                  reinterpret_cast<const uint32_t*>(S.vz), S.pid};
+  uint32_t* const dst[7] = {S.cell_b, reinterpret_cast<uint32_t*>(S.fx_b), reinterpret_cast<uint32_t*>(S.fy_b),
+                            reinterpret_cast<uint32_t*>(S.vx_b), reinterpret_cast<uint32_t*>(S.vy_b),
+                            reinterpret_cast<uint32_t*>(S.vz_b), S.pid_b};
+  for (int64_t c0 = (int64_t)blockIdx.x * kBandChunk; c0 < n; c0 += (int64_t)gridDim.x * kBandChunk) {
+    const int m = (int)min((int64_t)kBandChunk, n - c0);
+    uint32_t v[7][kBandPer];
+#pragma unroll
+    for (int f = 0; f < 7; ++f)
+#pragma unroll
+      for (int u = 0; u < kBandPer; ++u) {
+        const int k = t + u * kBandThreads;
+        v[f][u] = k < m ? __ldcs(src[f] + c0 + k) : 0u;
+      }
+    for (int b = t; b <= nb; b += kBandThreads) h[b] = 0;
+    __syncthreads();
+    int band[kBandPer], at[kBandPer];
+#pragma unroll
+    for (int u = 0; u < kBandPer; ++u) {
+      band[u] = t + u * kBandThreads < m ? band_of(v[0][u], ncy, nb) : -1;
+      at[u] = band[u] >= 0 ? atomicAdd(&h[band[u]], 1) : 0;
+    }
+    __syncthreads();
+    if (t < 32) {   // exclusive scan of the bands' counts
+      int a[kBandSums], sum = 0;
+#pragma unroll
+      for (int q = 0; q < kBandSums; ++q) {
+        const int b = t * kBandSums + q;
+        a[q] = sum;
+        sum += b <= nb ? h[b] : 0;
+      }
+      int incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (t >= o) incl += y;
+      }
+#pragma unroll
+      for (int q = 0; q < kBandSums; ++q) off[t * kBandSums + q] = a[q] + incl - sum;
+    } else {
+      for (int b = t - 32; b <= nb; b += kBandThreads - 32) base[b] = h[b] ? atomicAdd(S.scratch2 + b, h[b]) : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kBandPer; ++u)
+      if (band[u] >= 0) {
+        const int r = at[u];
+        at[u] = off[band[u]] + r;
+        place[at[u]] = base[band[u]] + r;
+      }
+#pragma unroll
+    for (int f = 0; f < 7; ++f) {
+#pragma unroll
+      for (int u = 0; u < kBandPer; ++u)
+        if (band[u] >= 0) stage[f & 1][at[u]] = v[f][u];
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < kBandPer; ++u) {
+        const int k = t + u * kBandThreads;
+        if (k < m) dst[f][place[k]] = stage[f & 1][k];
+      }
+    }
+    __syncthreads();
+  }
+}
+
 template <typename T>
 __device__ __forceinline__ void swp(T*& a, T*& b) { T* t = a; a = b; b = t; }
 
@@ -263,6 +403,15 @@ __global__ void sort_swap(SlotDev* slots, const uint8_t* mask, int nslots) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nslots || !mask[s]) return;
   SlotDev& S = slots[s];
+  swp(S.cell, S.cell_b); swp(S.fx, S.fx_b); swp(S.fy, S.fy_b);
+  swp(S.vx, S.vx_b); swp(S.vy, S.vy_b); swp(S.vz, S.vz_b); swp(S.pid, S.pid_b);
+}
+
+__global__ void sort_band_swap(const JobDev* jobs, SlotDev* slots, const int* counts, const uint8_t* mask, int nslots) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= nslots || !mask[s]) return;
+  SlotDev& S = slots[s];
+  if (!banded_slot(jobs[S.job], counts[s])) return;
   swp(S.cell, S.cell_b); swp(S.fx, S.fx_b); swp(S.fy, S.fy_b);
   swp(S.vx, S.vx_b); swp(S.vy, S.vy_b); swp(S.vz, S.vz_b); swp(S.pid, S.pid_b);
 }
@@ -296,7 +445,7 @@ int launch_sort_mask(const EngineLaunch& L, uint8_t* mask, int offset, cudaStrea
 }
 
 int launch_sort(const EngineLaunch& L, uint8_t* mask, int max_cells, int max_particles, bool by_disorder,
-                cudaStream_t st) {
+                bool random_order, cudaStream_t st) {
   if (L.nslots == 0) return 0;
   const int ncells = max_cells + 1;
   const int ntiles = (ncells + kTile - 1) / kTile;
@@ -306,9 +455,18 @@ int launch_sort(const EngineLaunch& L, uint8_t* mask, int max_cells, int max_par
   sort_hist<<<dim3(gp, L.nslots), 256, 0, st>>>(L.jobs, L.slots, L.counts, mask, L.aux, by_disorder ? 1 : 0);
   if (by_disorder) sort_filter_kernel<<<(L.nslots + 255) / 256, 256, 0, st>>>(mask, L.counts, L.aux, L.nslots);
   sort_tile_sums<<<dim3(std::min(ntiles, 4 * L.num_sms), L.nslots), 256, 0, st>>>(L.jobs, L.slots, mask);
-  sort_scan_parts<<<L.nslots, 256, 0, st>>>(L.jobs, L.slots, mask);
+  sort_scan_parts<<<L.nslots, 256, 0, st>>>(L.jobs, L.slots, mask, L.aux);
   sort_apply<<<dim3(std::min(ntiles, 4 * L.num_sms), L.nslots), 256, 0, st>>>(L.jobs, L.slots, mask);
-  sort_scatter<<<dim3(gp, L.nslots), 256, 0, st>>>(L.jobs, L.slots, L.counts, mask);
+  int k = 0;
+  if (random_order && max_particles >= kBandMinParticles) {
+    const int gb = std::min((max_particles + kBandChunk - 1) / kBandChunk, 4 * L.num_sms);
+    sort_band_init<<<L.nslots, 128, 0, st>>>(L.jobs, L.slots, L.counts, mask);
+    sort_band_scatter<<<dim3(gb, L.nslots), kBandThreads, 0, st>>>(L.jobs, L.slots, L.counts, mask);
+    sort_band_swap<<<(L.nslots + 255) / 256, 256, 0, st>>>(L.jobs, L.slots_mut, L.counts, mask, L.nslots);
+    k = 3;
+  }
+  const int gs = std::min(gp, kScatterCtas * L.num_sms);
+  sort_scatter<<<dim3(gs, L.nslots), 256, 0, st>>>(L.jobs, L.slots, L.counts, mask, L.aux);
   sort_swap<<<(L.nslots + 255) / 256, 256, 0, st>>>(L.slots_mut, mask, L.nslots);
-  return by_disorder ? 8 : 7;
+  return k + (by_disorder ? 8 : 7);
 }
