@@ -459,6 +459,7 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   int max_depth = 0, max_cycles = 1, nu_pre_max = 1, nu_post_max = 1;
   int nu_pre_min = 1 << 30, nu_post_min = 1 << 30;
   size_t coarse_smem = 0;
+  int coarse_side = 0;
   for (int id : ids) {
     const JobHost& J = E->jobs[id];
     const JobDev& D = J.dev;
@@ -487,6 +488,7 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
       cluster_smem = std::max(cluster_smem, mg_cluster_smem(D.nl, D.lc, D.levels, E->cluster_C));
     } else {
       coarse.push_back(id);
+      coarse_side = std::max(coarse_side, D.nl[D.lc]);
       coarse_smem = std::max(coarse_smem, mg_coarse_smem(D.nl, D.lc, D.levels));
     }
   }
@@ -556,6 +558,7 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   M.cluster_smem = cluster_smem;
   M.max_depth = max_depth;
   M.coarse_smem = coarse_smem;
+  M.coarse_side = coarse_side;
   M.nu_pre_max = nu_pre_max;
   M.nu_post_max = nu_post_max;
   M.pdl = E->pdl ? 1 : 0;

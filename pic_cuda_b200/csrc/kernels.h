@@ -78,6 +78,7 @@ struct MgLaunch {
   size_t cluster_smem;
   int max_depth;                                         // max lc over jobs
   size_t coarse_smem;
+  int coarse_side;                                       // largest first level of the single-CTA coarse solves
   int nu_pre_max, nu_post_max;                           // shared-memory sizing of the tile kernels
   int fast_nu_pre, fast_nu_post;                         // smoothing counts shared by every job, else -1
   int pdl;                                               // programmatic dependent launches in the V-cycle

@@ -27,6 +27,7 @@
 #include <algorithm>
 #include "common.cuh"
 #include "kernels.h"
+#include "mg_coarse.cuh"
 #include "mg_strips.cuh"
 #include "mg_tiles.h"
 #include "tma.cuh"
@@ -1379,8 +1380,12 @@ int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, cudaStream_t s) {
   for (int l = 0; l < M.max_depth; ++l)
     if (M.n_down[l]) { prev_fast = launch_down(M, l, L, prev_fast, s); ++k; }
   if (M.n_coarse) {
-    launch_k(mg_coarse_kernel, M.n_coarse, kCoarseThreads, M.coarse_smem, prev_fast && M.pdl, s, M.coarse_jobs,
-             L.jobs, L.st);
+    if (M.coarse_side <= mgc::kTop)
+      launch_k(mgc::mg_coarse_reg_kernel, M.n_coarse, mgc::kThreads, 0, prev_fast && M.pdl, s, M.coarse_jobs, L.jobs,
+               (const JobState*)L.st);
+    else
+      launch_k(mg_coarse_kernel, M.n_coarse, kCoarseThreads, M.coarse_smem, prev_fast && M.pdl, s, M.coarse_jobs,
+               L.jobs, (const JobState*)L.st);
     prev_fast = true;
     ++k;
   }
