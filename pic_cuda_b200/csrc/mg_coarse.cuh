@@ -15,7 +15,11 @@
 // kernel, and code that is unrolled by level (tried: 42 k cycles instead of the shared-memory solver's
 // 29 k with stamps) waits for its instructions.
 // Same expressions in the same order at every node as the shared-memory solver (coarse_solve), so
-// the results are the same bits.
+// the results are the same bits.  Measured on B200, from f in memory to the stored correction of 65^2 .. 3^2 at
+// 2 + 2 sweeps: 29.4 k cycles with the shared-memory solver, 19.0 k here (a half-sweep of 65^2 410, of 33^2 270,
+// of the others 180-200: one shared access, one shuffle, seven dependent operations and a barrier);
+// V-cycle at 129^2 28.6 -> 22.4 us, at 1025^2 63.4 -> 56.6 us.  Tables of the levels' places in shared memory in
+// place of the selects below were slower (24.4 us).
 #pragma once
 #include "common.cuh"
 #include "mg_strips.cuh"
@@ -38,15 +42,17 @@ __host__ __device__ constexpr int offset_of(int k) {
   return o;
 }
 
-struct Shared {
+struct __align__(16) Shared {
   // 65^2: the first and last row of every warp's four, by column of the pair: [first, last][column][1 +
   // warp][lane], zero beyond the grid; and the first row's residuals
   float edge[2][2][18][32];
-  float res[2][18][33];
   // the other levels' corrections, right-hand sides and residuals of odd rows
-  float e[offset_of(kPairs)], f[offset_of(kPairs)], r[offset_of(kPairs)];
+  float e[(offset_of(kPairs) + 3) & ~3];
+  float f[offset_of(kPairs)], r[offset_of(kPairs)];
+  float res[2][18][33];
   float h2[6], ih2[6];   // 65^2 .. 3^2
 };
+constexpr int kZeroed = (sizeof(Shared::edge) + sizeof(Shared::e)) / 16;   // what starts as zero comes first
 
 struct Params {
   float omega, om1;
@@ -248,9 +254,8 @@ __global__ void __launch_bounds__(kThreads) mg_coarse_reg_kernel(const int* __re
   A.bottom = top + J.levels - 1 - lc;
   float* const e = J.e[lc];
   const float* const f = (lc == 0 && st[job].fsel) ? J.f0b : J.f[lc];
-  // shared arrays start as zero: grid boundaries, and corrections that no sweep touches
-  for (int k = t; k < (int)(sizeof(Shared) / 4); k += kThreads) reinterpret_cast<float*>(&S)[k] = 0.f;
-  __syncthreads();
+  // zero: the grid boundaries, and corrections that no sweep touches
+  for (int k = t; k < kZeroed; k += kThreads) reinterpret_cast<float4*>(&S)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (t < 6) {
     // constants of side 2^(6 - t) + 1, which is level lc + t - (top + 1)
     const double hl = J.h * (double)(1 << (lc + max(0, t - 1 - top)));

@@ -17,7 +17,9 @@
 //              then residual + full weighting straight from shared memory
 //   On levels with enough nodes (strip_rows, engine.cu) both legs run as pipelines of rows in
 //   registers instead of tiles (mg_strips.cuh), with the same bits.
-//   mg_coarse  one CTA per job runs the whole V-cycle from <= 65x65 down in shared memory
+//   mg_coarse  one CTA per job runs the whole V-cycle from <= 65x65 down with the nodes in
+//              registers (mg_coarse.cuh), from a larger first level (PIC_OPT_MG_COARSE_TOP) in
+//              shared memory
 //   (opt-in: levels up to 257^2 or 513^2 in one thread-block cluster, mg_cluster.cu)
 //   mg_up      prolongation + nu_post sweeps on 32x32 tiles; on level 0 also the FP64
 //              update phi += e, the new FP64 residual and the tile's partial norm;
