@@ -148,16 +148,6 @@ __global__ void efield_f64_kernel(const double* __restrict__ phi, double* __rest
   }
 }
 
-__global__ void step_begin_kernel(JobState* st, const JobDev* jobs, int njobs, const uint8_t* job_mask) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= njobs || (job_mask && !job_mask[j])) return;
-  JobState& T = st[j];
-  for (int s = 0; s < PIC_MAX_SPECIES; ++s) {
-    T.ke[s] = 0.0;
-    for (int q = 0; q < 8; ++q) T.collisions[s][q] = 0ull;
-  }
-}
-
 // Before a flush pass (the pending kick and collisions of the last step, applied ahead of a
 // read-back): the kinetic energy of the jobs it applies to restarts, so that afterwards it is
 // the energy of the velocities the read-back returns.
@@ -196,17 +186,6 @@ __global__ void rho_sum_final_kernel(const JobDev* __restrict__ jd, const double
     double s = 0.0;
     for (int k = 0; k < nparts; ++k) s += part[k];
     st->total_charge = s * jd->qref;
-  }
-}
-
-__global__ void zero_rho_all_kernel(const JobDev* __restrict__ jobs, int njobs) {
-  const JobDev& J = jobs[blockIdx.y];
-  if (J.nslots == 0 && J.nx == 0) return;
-  const int64_t N = (int64_t)J.nx * J.ny;
-  if (J.deposit_mode == 0 && J.rho_f) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N; k += (int64_t)gridDim.x * blockDim.x) J.rho_f[k] = 0.f;
-  } else if (J.deposit_mode == 1 && J.rho_i) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N; k += (int64_t)gridDim.x * blockDim.x) J.rho_i[k] = 0;
   }
 }
 
@@ -262,20 +241,9 @@ int launch_ke_reset_pending(JobState* st, int njobs, cudaStream_t s) {
   ke_reset_pending_kernel<<<(njobs + 127) / 128, 128, 0, s>>>(st, njobs);
   return 1;
 }
-int launch_step_begin(JobState* st, const JobDev* jobs, int njobs, const uint8_t* job_mask, cudaStream_t s) {
-  if (!njobs) return 0;
-  step_begin_kernel<<<(njobs + 127) / 128, 128, 0, s>>>(st, jobs, njobs, job_mask);
-  return 1;
-}
 int launch_step_end(JobState* st, int njobs, const uint8_t* job_mask, int set_pending, int advance, cudaStream_t s) {
   if (!njobs) return 0;
   step_end_kernel<<<(njobs + 127) / 128, 128, 0, s>>>(st, njobs, job_mask, set_pending, advance);
-  return 1;
-}
-int launch_zero_rho_all(const EngineLaunch& L, int max_nodes, cudaStream_t s) {
-  if (!L.njobs) return 0;
-  const int gx = (int)std::min<int64_t>(std::max<int64_t>(((int64_t)max_nodes + 1023) / 1024, 1), 1024);
-  zero_rho_all_kernel<<<dim3(gx, L.njobs), 256, 0, s>>>(L.jobs, L.njobs);
   return 1;
 }
 void launch_rho_sum(const JobDev* jd, JobState* st, double* scratch, int nparts, cudaStream_t s) {

@@ -589,6 +589,13 @@ std::vector<int> alive_ids(pic_engine* E) {
   return v;
 }
 
+// Can any job's step create particles?  (The launch that appends them is left out where none can.)
+bool any_ionization(pic_engine* E) {
+  for (int j = 0; j < E->njobs_hw; ++j)
+    if (E->jobs[j].alive && has_ionization(E->jobs[j].cfg)) return true;
+  return false;
+}
+
 int ensure_mg_all(pic_engine* E) {
   if (!E->mg_dirty && E->mg_all.valid) return PIC_OK;
   const int rc = build_mg(E, alive_ids(E), E->mg_all);
@@ -604,11 +611,11 @@ int ensure_mg_all(pic_engine* E) {
 int solve(pic_engine* E, const MgBuild& B, const uint8_t* active, cudaStream_t s) {
   if (!B.valid) return PIC_OK;
   EngineLaunch L = make_launch(E, active);
-  E->launches += launch_mg_init(L, B.L, s);
+  E->launches += launch_mg_init(L, B.L, nullptr, s);
   const int unchecked = std::max(1, std::min(E->last_solve_cycles - 1, B.max_cycles));
   int c = 0;
   for (; c < B.max_cycles; ++c) {
-    E->launches += launch_mg_vcycle(L, B.L, s);
+    E->launches += launch_mg_vcycle(L, B.L, nullptr, s);
     E->vcycles++;
     if (c + 1 < unchecked) continue;
     CK(cudaMemcpyAsync(E->h_pinned, E->d_running, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -672,7 +679,7 @@ int flush(pic_engine* E, cudaStream_t s, int job = -1) {
   }
   EngineLaunch L = make_launch(E, active);
   E->launches += launch_ke_reset_pending(st, nst, s);
-  E->launches += launch_mover(L, PIC_PHASE_KICK_I | PIC_PHASE_MCC_I | PIC_PHASE_GATED_I, 0, s);
+  E->launches += launch_mover(L, PIC_PHASE_KICK_I | PIC_PHASE_MCC_I | PIC_PHASE_GATED_I, 0, false, s);
   E->launches += launch_ionize(L, false, s);
   E->launches += launch_step_end(st, nst, nullptr, 0, 0, s);
   for (int j = 0; j < E->njobs_hw; ++j)
@@ -736,11 +743,7 @@ int step_once(pic_engine* E, cudaStream_t s) {
   bool sorted = false;
   int rc = sort_jobs(E, L, sort_before_first, s, &sorted);
   if (rc) return rc;
-  E->launches += launch_step_begin(E->d_st, E->d_jobs, E->njobs_hw, nullptr, s);
-  int max_nodes = 0;
-  for (int j = 0; j < E->njobs_hw; ++j)
-    if (E->jobs[j].alive) max_nodes = std::max(max_nodes, E->jobs[j].dev.nx * E->jobs[j].dev.ny);
-  E->launches += launch_zero_rho_all(L, max_nodes, s);
+  E->launches += launch_step_head(L, s);
   if (E->profile) {
     if (E->mover_events_used == E->mover_events.size()) {
       std::pair<cudaEvent_t, cudaEvent_t> ev;
@@ -753,11 +756,11 @@ int step_once(pic_engine* E, cudaStream_t s) {
     E->mover_events_used++;
   }
   E->launches += launch_mover(L, PIC_PHASE_KICK_I | PIC_PHASE_MCC_I | PIC_PHASE_DRIFT_I | PIC_PHASE_WALLS_I |
-                                     PIC_PHASE_DEPOSIT_I | PIC_PHASE_GATED_I, 0, s);
+                                     PIC_PHASE_DEPOSIT_I | PIC_PHASE_GATED_I, 0, true, s);
   L.ev_mover_begin = L.ev_mover_end = nullptr;
   // the pairs of this step's ionisations (appended after the live particles, drifted and
   // deposited) before the field solve, which needs their charge
-  E->launches += launch_ionize(L, true, s);
+  if (any_ionization(E)) E->launches += launch_ionize(L, true, s);
   // removal of the absorbed particles, then the sort due before the next step, on the side
   // stream while the field is solved (they touch only particle arrays, the solve only grids)
   CK(cudaEventRecord(E->ev_fork, s));
@@ -792,16 +795,12 @@ int build_step_graph(pic_engine* E, bool with_sort, cudaGraphExec_t* out, int64_
   CK(cudaGraphCreate(&g, 0));
   EngineLaunch L = make_launch(E, nullptr);
   int64_t n = 0;
-  int max_nodes = 0;
-  for (int j = 0; j < E->njobs_hw; ++j)
-    if (E->jobs[j].alive) max_nodes = std::max(max_nodes, E->jobs[j].dev.nx * E->jobs[j].dev.ny);
   cudaError_t err = cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (err != cudaSuccess) { cudaGraphDestroy(g); return fail(PIC_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(err)); }
-  n += launch_step_begin(E->d_st, E->d_jobs, E->njobs_hw, nullptr, s);
-  n += launch_zero_rho_all(L, max_nodes, s);
+  n += launch_step_head(L, s);
   n += launch_mover(L, PIC_PHASE_KICK_I | PIC_PHASE_MCC_I | PIC_PHASE_DRIFT_I | PIC_PHASE_WALLS_I | PIC_PHASE_DEPOSIT_I |
-                           PIC_PHASE_GATED_I, 0, s);
-  n += launch_ionize(L, true, s);
+                           PIC_PHASE_GATED_I, 0, true, s);
+  if (any_ionization(E)) n += launch_ionize(L, true, s);
   // removal of the absorbed particles and the sort due before the next step, on a parallel
   // branch of the graph beside the solve
   if (err == cudaSuccess) err = cudaEventRecord(E->ev_fork, s);
@@ -820,8 +819,7 @@ int build_step_graph(pic_engine* E, bool with_sort, cudaGraphExec_t* out, int64_
     n += launch_sort(L, E->d_mask, max_cells, (int)std::min<int64_t>(max_p, 1 << 30), true, false, E->side_stream);
   }
   if (err == cudaSuccess) err = cudaEventRecord(E->ev_join, E->side_stream);
-  n += launch_mg_init(L, E->mg_all.L, s);
-  cudaMemsetAsync(E->d_loop, 0, sizeof(int), s);
+  n += launch_mg_init(L, E->mg_all.L, E->d_loop, s);
   // conditional WHILE node for the V-cycles
   cudaStreamCaptureStatus cs;
   cudaGraph_t cg = nullptr;
@@ -845,9 +843,8 @@ int build_step_graph(pic_engine* E, bool with_sort, cudaGraphExec_t* out, int64_
     err = cudaStreamBeginCaptureToGraph(E->body_stream, bg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (err == cudaSuccess) {
       EngineLaunch LB = L;
-      body += launch_mg_vcycle(LB, E->mg_all.L, E->body_stream);
-      body += launch_vcycle_condition(h, E->d_running, E->d_loop, E->mg_all.max_cycles, E->d_loop_total,
-                                      E->body_stream);
+      const VcycleLoop loop{h, E->d_loop, E->mg_all.max_cycles, E->d_loop_total, E->d_loop + 1};
+      body += launch_mg_vcycle(LB, E->mg_all.L, &loop, E->body_stream);
       cudaGraph_t tmp = nullptr;
       err = cudaStreamEndCapture(E->body_stream, &tmp);
     }
@@ -977,6 +974,7 @@ int pic_engine_create(int device, int64_t pool_bytes, pic_engine** out) {
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&E->ev_fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&E->ev_join, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc(&E->d_loop, sizeof(int) * 4);
+  if (e == cudaSuccess) e = cudaMemset(E->d_loop, 0, sizeof(int) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&E->d_loop_total, sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMemset(E->d_loop_total, 0, sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMemset(E->d_counts, 0, sizeof(int) * nslots);
@@ -1629,7 +1627,7 @@ int pic_job_run_phases(pic_engine* E, int job, int flags, int64_t step_index, vo
   if (rc) return rc;
   if (flags & PIC_PHASE_WALLS) CK(cudaMemsetAsync(E->d_hits + job * kSlotsPerJob, 0, sizeof(int) * kSlotsPerJob, s));
   EngineLaunch L = make_launch(E, E->d_mask);
-  launch_mover(L, flags & 31, (uint32_t)step_index, s);
+  launch_mover(L, flags & 31, (uint32_t)step_index, false, s);
   if (flags & PIC_PHASE_MCC) launch_ionize(L, (flags & PIC_PHASE_DRIFT) != 0, s);
   CK(cudaStreamSynchronize(s));
   CK(cudaGetLastError());

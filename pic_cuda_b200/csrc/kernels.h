@@ -42,7 +42,10 @@ struct EngineLaunch {
 };
 
 int mover_blocks_per_sm();
-int launch_mover(const EngineLaunch& L, int flags, uint32_t explicit_step, cudaStream_t s);
+// Before a full step's particle pass: the node field, zero charge, reset diagnostics, work items.
+int launch_step_head(const EngineLaunch& L, cudaStream_t s);
+// after_head: launch_step_head ran before it (the pass needs neither the node field nor the items).
+int launch_mover(const EngineLaunch& L, int flags, uint32_t explicit_step, bool after_head, cudaStream_t s);
 int launch_compact(const EngineLaunch& L, cudaStream_t s);
 int launch_ionize(const EngineLaunch& L, bool drift_and_deposit, cudaStream_t s);
 // Counting sort of the slots in sort_mask; by_disorder: the histogram pass also counts the
@@ -51,14 +54,10 @@ int launch_ionize(const EngineLaunch& L, bool drift_and_deposit, cudaStream_t s)
 // random_order: the particles were loaded since the last sort, so large slots take the band pass.
 int launch_sort(const EngineLaunch& L, uint8_t* sort_mask, int max_cells, int max_particles, bool by_disorder,
                 bool random_order, cudaStream_t s);
-int launch_step_begin(JobState* st, const JobDev* jobs, int njobs, const uint8_t* job_mask, cudaStream_t s);
 int launch_ke_reset_pending(JobState* st, int njobs, cudaStream_t s);
 int launch_step_end(JobState* st, int njobs, const uint8_t* job_mask, int set_pending, int advance, cudaStream_t s);
 void launch_pid_max(const SlotDev* slot_dev, int64_t n, JobState* st, cudaStream_t s);
-int launch_zero_rho_all(const EngineLaunch& L, int max_nodes, cudaStream_t s);
 int launch_sort_mask(const EngineLaunch& L, uint8_t* mask, int offset, cudaStream_t s);
-int launch_vcycle_condition(cudaGraphConditionalHandle h, const int* running, int* iterations, int max_iterations,
-                            unsigned long long* total, cudaStream_t s);
 void launch_rho_sum(const JobDev* jd, JobState* st, double* scratch, int nparts, cudaStream_t s);
 
 // Multigrid (all jobs of a launch at once).
@@ -107,8 +106,17 @@ int mg_strip_rows(int leg, int nu, int level, int at_most);
 // Grid size (0: not available) and shared memory of the cooperative levels kernel.
 int mg_levels_configure(int num_sms, int nu_pre_max, int nu_post_max, size_t coarse_smem, size_t* smem,
                         size_t* quarter_floats);
-int launch_mg_init(const EngineLaunch& L, const MgLaunch& M, cudaStream_t s);
-int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, cudaStream_t s);
+// loop: iteration count of a step graph's V-cycle loop, zeroed here (may be null).
+int launch_mg_init(const EngineLaunch& L, const MgLaunch& M, int* loop, cudaStream_t s);
+// cond: the V-cycle is the body of a step graph's WHILE node, and ends by setting its condition.
+struct VcycleLoop {
+  cudaGraphConditionalHandle handle;
+  int* iterations;
+  int max_iterations;
+  unsigned long long* total;
+  int* ticket;                 // jobs that have finished this cycle (zero between cycles)
+};
+int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, const VcycleLoop* cond, cudaStream_t s);
 void mg_configure_coarse(size_t smem_bytes);
 // Shared memory of the one-CTA coarse solver for levels lc .. levels-1.
 size_t mg_coarse_smem(const int* nl, int lc, int levels);

@@ -169,25 +169,71 @@ __device__ void collide(const JobDev& J, const SlotDev& S, const SlotDev* slots,
   atomicAdd(&proc_count[chosen & 7], 1u);
 }
 
-// E per unit cell (-dphi across one cell) at every node of every job, from the job's
-// current FP64 potential with the computeElectricField stencils (kernels.cu:134-191):
-// (phi[i-1] - phi[i+1]) / 2 inside, phi[i] - phi[i+1] on the first and phi[i-1] - phi[i]
-// on the last node of a row, the same along columns; rounded to FP32 once.  Job j uses
-// blockIdx.y == j and a grid-stride loop over its nodes.
+// E per unit cell (-dphi across one cell) at node k of a job, from its current FP64 potential with the
+// computeElectricField stencils (kernels.cu:134-191): (phi[i-1] - phi[i+1]) / 2 inside, phi[i] -
+// phi[i+1] on the first and phi[i-1] - phi[i] on the last node of a row, the same along columns;
+// rounded to FP32 once.
+__device__ __forceinline__ float2 efield_at(const double* __restrict__ phi, int nx, int ny, int k) {
+  const int j = k / nx, i = k - j * nx;
+  const int il = i > 0 ? i - 1 : 0, ir = i < nx - 1 ? i + 1 : nx - 1;
+  const int jl = j > 0 ? j - 1 : 0, jr = j < ny - 1 ? j + 1 : ny - 1;
+  const double sx = (i > 0 && i < nx - 1) ? 0.5 : 1.0, sy = (j > 0 && j < ny - 1) ? 0.5 : 1.0;
+  const double ex = (phi[j * nx + il] - phi[j * nx + ir]) * sx;
+  const double ey = (phi[jl * nx + i] - phi[jr * nx + i]) * sy;
+  return make_float2((float)ex, (float)ey);
+}
+
+// The node field of every job.  Job j uses blockIdx.y == j and a grid-stride loop over its nodes.
 __global__ void __launch_bounds__(256) efield32_kernel(const JobDev* __restrict__ jobs, const JobState* __restrict__ st) {
   const JobDev& J = jobs[blockIdx.y];
   float2* const out = J.efield;
   if (!out) return;
   const double* __restrict__ phi = J.phi64[st[blockIdx.y].phi_cur];
   const int nx = J.nx, ny = J.ny, N = nx * ny;
+  for (int k = blockIdx.x * 256 + threadIdx.x; k < N; k += gridDim.x * 256) out[k] = efield_at(phi, nx, ny, k);
+}
+
+// Exclusive prefix of mover work items (kItem particles) per active slot, by one thread.
+__device__ void item_prefix_of(const int* __restrict__ counts, const uint8_t* __restrict__ active, int* prefix,
+                               int nslots) {
+  int a = 0;
+  for (int s = 0; s < nslots; ++s) {
+    prefix[s] = a;
+    if (!active || active[s]) a += (counts[s] + kItem - 1) / kItem;
+  }
+  prefix[nslots] = a;
+}
+__global__ void chunk_table_kernel(const int* __restrict__ counts, const uint8_t* __restrict__ active,
+                                   int* __restrict__ chunk_prefix, int nslots) {
+  if (threadIdx.x == 0) item_prefix_of(counts, active, chunk_prefix, nslots);
+}
+
+// What a full step does before its particle pass, in one launch: the node field of every job, its charge
+// grid zeroed, the step's diagnostics reset and the work items counted.  (Four launches of 2-4 us each
+// before, most of it launch latency on small jobs: 129^2 step 123 -> 108 us together with the merged
+// V-cycle end and the memsets that moved into the solver's kernels.)
+__global__ void __launch_bounds__(256) step_head_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st,
+                                                        const int* __restrict__ counts,
+                                                        const uint8_t* __restrict__ active, int* __restrict__ prefix,
+                                                        int nslots) {
+  const JobDev& J = jobs[blockIdx.y];
+  if (blockIdx.x == gridDim.x - 1) {   // the block with the fewest nodes
+    if (blockIdx.y == 0 && threadIdx.x == 0) item_prefix_of(counts, active, prefix, nslots);
+    JobState& T = st[blockIdx.y];
+    const int t = (int)threadIdx.x - 32;
+    if (t >= 0 && t < PIC_MAX_SPECIES) T.ke[t] = 0.0;
+    if (t >= 32 && t < 32 + 8 * PIC_MAX_SPECIES) T.collisions[(t - 32) >> 3][(t - 32) & 7] = 0ull;
+  }
+  float2* const out = J.efield;
+  if (!out) return;                    // no such job
+  const double* __restrict__ phi = J.phi64[st[blockIdx.y].phi_cur];
+  const int nx = J.nx, ny = J.ny, N = nx * ny;
+  float* const rf = J.deposit_mode == 0 ? J.rho_f : nullptr;
+  long long* const ri = J.deposit_mode == 1 ? J.rho_i : nullptr;
   for (int k = blockIdx.x * 256 + threadIdx.x; k < N; k += gridDim.x * 256) {
-    const int j = k / nx, i = k - j * nx;
-    const int il = i > 0 ? i - 1 : 0, ir = i < nx - 1 ? i + 1 : nx - 1;
-    const int jl = j > 0 ? j - 1 : 0, jr = j < ny - 1 ? j + 1 : ny - 1;
-    const double sx = (i > 0 && i < nx - 1) ? 0.5 : 1.0, sy = (j > 0 && j < ny - 1) ? 0.5 : 1.0;
-    const double ex = (phi[j * nx + il] - phi[j * nx + ir]) * sx;
-    const double ey = (phi[jl * nx + i] - phi[jr * nx + i]) * sy;
-    out[k] = make_float2((float)ex, (float)ey);
+    out[k] = efield_at(phi, nx, ny, k);
+    if (rf) rf[k] = 0.f;
+    else if (ri) ri[k] = 0;
   }
 }
 
@@ -636,19 +682,6 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
   flush();
 }
 
-// Exclusive prefix of mover work items (kItem particles) per active slot.
-__global__ void chunk_table_kernel(const int* __restrict__ counts, const uint8_t* __restrict__ active,
-                                   int* __restrict__ chunk_prefix, int nslots) {
-  if (threadIdx.x == 0) {
-    int a = 0;
-    for (int s = 0; s < nslots; ++s) {
-      chunk_prefix[s] = a;
-      if (!active || active[s]) a += (counts[s] + kItem - 1) / kItem;
-    }
-    chunk_prefix[nslots] = a;
-  }
-}
-
 int mover_blocks_per_sm() {
   cudaFuncSetAttribute(mover_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMoverSmem);
   int b = 0;
@@ -660,15 +693,25 @@ int mover_blocks_per_sm() {
   return b;
 }
 
-int launch_mover(const EngineLaunch& L, int flags, uint32_t explicit_step, cudaStream_t stream) {
-  int k = 2;
-  if ((flags & PIC_PHASE_KICK_I) && L.njobs > 0) {
-    // the node field of every job's current potential, for the kick
-    const int gx = std::max(1, std::min(4096, 8 * L.num_sms / L.njobs));
-    efield32_kernel<<<dim3(gx, L.njobs), 256, 0, stream>>>(L.jobs, L.st);
+int launch_step_head(const EngineLaunch& L, cudaStream_t stream) {
+  if (!L.njobs) return 0;
+  const int gx = std::max(1, std::min(4096, 8 * L.num_sms / L.njobs));
+  step_head_kernel<<<dim3(gx, L.njobs), 256, 0, stream>>>(L.jobs, L.st, L.counts, L.active, L.chunk_prefix, L.nslots);
+  return 1;
+}
+
+int launch_mover(const EngineLaunch& L, int flags, uint32_t explicit_step, bool after_head, cudaStream_t stream) {
+  int k = 1;
+  if (!after_head) {
+    if ((flags & PIC_PHASE_KICK_I) && L.njobs > 0) {
+      // the node field of every job's current potential, for the kick
+      const int gx = std::max(1, std::min(4096, 8 * L.num_sms / L.njobs));
+      efield32_kernel<<<dim3(gx, L.njobs), 256, 0, stream>>>(L.jobs, L.st);
+      ++k;
+    }
+    chunk_table_kernel<<<1, 32, 0, stream>>>(L.counts, L.active, L.chunk_prefix, L.nslots);
     ++k;
   }
-  chunk_table_kernel<<<1, 32, 0, stream>>>(L.counts, L.active, L.chunk_prefix, L.nslots);
   if (L.ev_mover_begin) cudaEventRecord(L.ev_mover_begin, stream);
   mover_kernel<<<L.mover_grid, PIC_MOVER_THREADS, kMoverSmem, stream>>>(L.jobs, L.st, L.slots, L.counts,
                                                                           L.hit_counts, L.chunk_prefix, L.nslots, flags,

@@ -103,13 +103,18 @@ __device__ bool last_of_job(JobState& T, int nlocal) {
 // batch of asynchronous copies; the guess is formed once per node in shared memory.  The
 // same pass sums the deposited charge (deterministic per-tile partials, like the norms).
 __global__ void __launch_bounds__(256) mg_init_kernel(const TileRef* __restrict__ tiles, const JobDev* __restrict__ jobs,
-                                                      const JobState* __restrict__ st) {
+                                                      const JobState* __restrict__ st, int* running, int* loop) {
   constexpr int PW = kTI + 2, NT = 256;
   constexpr int NP = (PW * PW + NT - 1) / NT;
   constexpr int NO = kTI * kTI / NT;
   __shared__ __align__(16) double G[PW * PW];    // guess with halo (the current potential first)
   __shared__ __align__(16) double Q[PW * PW];    // previous solution with halo (warm start 1)
   __shared__ __align__(16) double RH[kTI * kTI]; // rho of the owned nodes, raw
+  // the solve's counters start at zero (mg_init_finish_kernel and the V-cycles come after this launch)
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *running = 0;
+    if (loop) *loop = 0;
+  }
   const TileRef tr = tiles[blockIdx.x];
   const JobDev& J = jobs[tr.job];
   const JobState& T = st[tr.job];
@@ -1114,27 +1119,47 @@ __global__ void __launch_bounds__(NT, MODE ? 5 : 1) mg_up_fast_kernel(const Tile
 // swaps the potential and defect buffers and takes a converged job out of the running count.  Launched after the
 // level-0 up kernel (waits for it in tma::pdl_wait); the next V-cycle's first launch waits for
 // this one.
+// In a step graph (loop.iterations set) the CTA of the last job also decides whether the V-cycle WHILE
+// node runs again: while any job is still iterating, at most max_iterations times per solve.
+__device__ __forceinline__ void loop_again(const VcycleLoop& loop, int running) {
+  const int it = ++(*loop.iterations);
+  *loop.total += 1ull;
+  cudaGraphSetConditional(loop.handle, (running > 0 && it < loop.max_iterations) ? 1u : 0u);
+}
+
 __global__ void __launch_bounds__(1024) mg_finish_kernel(const int* __restrict__ job_list,
                                                         const JobDev* __restrict__ jobs,
-                                                        JobState* __restrict__ st, int* running) {
+                                                        JobState* __restrict__ st, int* running, const VcycleLoop loop) {
   tma::pdl_trigger();
   tma::pdl_wait();
   const int job = job_list[2 * blockIdx.x], n = job_list[2 * blockIdx.x + 1];
   const JobDev& J = jobs[job];
   JobState& T = st[job];
-  if (T.converged) return;
-  const double r2 = ordered_sum(J.partials, n, 2, 0);
-  if (threadIdx.x != 0) return;
-  T.rnorm2 = r2;
-  T.relres = T.fnorm2 > 0.0 ? sqrt(r2 / T.fnorm2) : sqrt(r2);
-  T.cycles += 1;
-  const int cur = T.phi_cur;
-  T.phi_cur = T.phi_nxt;
-  T.phi_nxt = cur;
-  T.fsel ^= 1;
-  if (T.relres < J.tol) { T.converged = 1; atomicSub(running, 1); }
-  else if (T.cycles >= J.max_cycles) { T.converged = 2; atomicSub(running, 1); }
+  if (!T.converged) {
+    const double r2 = ordered_sum(J.partials, n, 2, 0);
+    if (threadIdx.x == 0) {
+      T.rnorm2 = r2;
+      T.relres = T.fnorm2 > 0.0 ? sqrt(r2 / T.fnorm2) : sqrt(r2);
+      T.cycles += 1;
+      const int cur = T.phi_cur;
+      T.phi_cur = T.phi_nxt;
+      T.phi_nxt = cur;
+      T.fsel ^= 1;
+      if (T.relres < J.tol) { T.converged = 1; atomicSub(running, 1); }
+      else if (T.cycles >= J.max_cycles) { T.converged = 2; atomicSub(running, 1); }
+    }
+  }
+  if (loop.iterations && threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(loop.ticket, 1) == (int)gridDim.x - 1) {
+      *loop.ticket = 0;
+      loop_again(loop, atomicAdd(running, 0));
+    }
+  }
 }
+
+// The same for V-cycles that do not end with mg_finish_kernel.
+__global__ void vcycle_condition_kernel(const int* running, const VcycleLoop loop) { loop_again(loop, *running); }
 
 // Launch with optional programmatic stream serialisation (the kernel may start while the
 // previous launch in the stream finishes; it waits in tma::pdl_wait before reading its output).
@@ -1272,10 +1297,13 @@ void mg_configure_coarse(size_t smem_bytes) {
   cudaFuncSetAttribute(mg_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)up_smem(16));
 }
 
-int launch_mg_init(const EngineLaunch& L, const MgLaunch& M, cudaStream_t s) {
-  cudaMemsetAsync(L.running, 0, sizeof(int), s);
-  if (!M.n_init) return 0;
-  mg_init_kernel<<<M.n_init, 256, 0, s>>>(M.init_tiles, L.jobs, L.st);
+int launch_mg_init(const EngineLaunch& L, const MgLaunch& M, int* loop, cudaStream_t s) {
+  if (!M.n_init) {
+    cudaMemsetAsync(L.running, 0, sizeof(int), s);
+    if (loop) cudaMemsetAsync(loop, 0, sizeof(int), s);
+    return 0;
+  }
+  mg_init_kernel<<<M.n_init, 256, 0, s>>>(M.init_tiles, L.jobs, L.st, L.running, loop);
   mg_init_finish_kernel<<<M.n_init_jobs, 1024, 0, s>>>(M.init_jobs, L.jobs, L.st, L.running);
   return 2;
 }
@@ -1327,7 +1355,7 @@ static bool launch_down(const MgLaunch& M, int l, const EngineLaunch& L, bool pd
   mg_down_kernel<<<M.n_down[l], 256, down_smem(M.nu_pre_max), s>>>(M.down_tiles[l], L.jobs, L.st, l);
   return false;
 }
-static bool launch_up(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, cudaStream_t s) {
+static bool launch_up(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, const VcycleLoop* cond, cudaStream_t s) {
   if (M.fast_nu_post < 0) {
     mg_up_kernel<<<M.n_up[l], 256, up_smem(M.nu_post_max), s>>>(M.up_tiles[l], L.jobs, L.st, l, l == 0 ? 1 : 0,
                                                                 L.running);
@@ -1342,12 +1370,21 @@ static bool launch_up(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl,
             L.st, l, l == 0 ? 1 : 0, s);
   }
   if (l == 0)
-    launch_k(mg_finish_kernel, M.n_finish, 1024, 0, M.pdl != 0, s, M.finish_jobs, L.jobs, L.st, L.running);
+    launch_k(mg_finish_kernel, M.n_finish, 1024, 0, M.pdl != 0, s, M.finish_jobs, L.jobs, L.st, L.running,
+             cond ? *cond : VcycleLoop{});
   return true;
 }
 
-int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, cudaStream_t s) {
+int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, const VcycleLoop* cond, cudaStream_t s) {
   int k = 0;
+  // the loop's condition in the last kernel where that is mg_finish_kernel, else after it
+  const bool fused = M.n_up[0] && M.fast_nu_post >= 0 && !M.n_upd;
+  auto end_loop = [&]() {
+    if (!cond || fused) return;
+    vcycle_condition_kernel<<<1, 1, 0, s>>>(L.running, *cond);
+    ++k;
+  };
+  const VcycleLoop* const up_cond = fused ? cond : nullptr;
   if (M.levels_grid > 0 && M.max_depth >= 2 && !M.n_cluster) {
     if (M.n_down[0]) { launch_down(M, 0, L, false, s); ++k; }
     MgLevelsArgs a{};
@@ -1372,8 +1409,9 @@ int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, cudaStream_t s) {
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, mg_levels_kernel, a);
     ++k;
-    if (M.n_up[0]) k += launch_up(M, 0, L, false, s) ? 2 : 1;   // + mg_finish_kernel
+    if (M.n_up[0]) k += launch_up(M, 0, L, false, up_cond, s) ? 2 : 1;   // + mg_finish_kernel
     if (M.n_upd) { mg_up_kernel<<<M.n_upd, 256, up_smem(0), s>>>(M.upd_tiles, L.jobs, L.st, 0, 2, L.running); ++k; }
+    end_loop();
     return k;
   }
   // every launch after the first may overlap its predecessor when both are compile-time-shape
@@ -1393,24 +1431,8 @@ int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, cudaStream_t s) {
   }
   if (M.n_cluster) { k += launch_mg_cluster(M.cluster_jobs, M.n_cluster, M.cluster_C, M.cluster_smem, L.jobs, L.st, s); prev_fast = false; }
   for (int l = M.max_depth - 1; l >= 0; --l)
-    if (M.n_up[l]) { prev_fast = launch_up(M, l, L, prev_fast, s); k += (prev_fast && l == 0) ? 2 : 1; }
+    if (M.n_up[l]) { prev_fast = launch_up(M, l, L, prev_fast, up_cond, s); k += (prev_fast && l == 0) ? 2 : 1; }
   if (M.n_upd) { mg_up_kernel<<<M.n_upd, 256, up_smem(0), s>>>(M.upd_tiles, L.jobs, L.st, 0, 2, L.running); ++k; }
+  end_loop();
   return k;
-}
-
-namespace {
-// Body-end kernel of the V-cycle WHILE node: loop again while any job is still iterating,
-// never more than max_iterations times per solve.
-__global__ void vcycle_condition_kernel(cudaGraphConditionalHandle h, const int* running, int* iterations,
-                                        int max_iterations, unsigned long long* total) {
-  const int it = ++(*iterations);
-  *total += 1ull;
-  cudaGraphSetConditional(h, (*running > 0 && it < max_iterations) ? 1u : 0u);
-}
-}  // namespace
-
-int launch_vcycle_condition(cudaGraphConditionalHandle h, const int* running, int* iterations, int max_iterations,
-                            unsigned long long* total, cudaStream_t s) {
-  vcycle_condition_kernel<<<1, 1, 0, s>>>(h, running, iterations, max_iterations, total);
-  return 1;
 }
