@@ -294,8 +294,8 @@ int pic_efield_f64(const double* phi, double* E_xy, int nx, int ny, double dx, d
  * than the fine one).  PIC_EMB_COARSEN_ANY takes the coarse kind from the 3x3 fine nodes as
  * the reference's comment at :73 states; PIC_EMB_PROLONG_BILINEAR prolongates bilinearly.
  * Stops when ||r|| / ||rhs|| over the FLUID nodes (||r|| / ||r_0|| if rhs is 0 there) is below
- * tol or after max_cycles V-cycles (PIC_ERR_NOT_CONVERGED); reading the norm synchronises
- * `stream` once per cycle.  tol == 0 runs exactly max_cycles V-cycles without reading it in
+ * tol or after max_cycles V-cycles (PIC_ERR_NOT_CONVERGED); `stream` is synchronised to read
+ * the norm at least once, and at most once per cycle.  tol == 0 runs exactly max_cycles V-cycles without reading it in
  * between (once at the end with relres_out) and, like pic_solve_multigrid_f64, returns
  * PIC_ERR_NOT_CONVERGED.  Working arrays come from a
  * per-device cache keyed by (nx, ny, levels); calls on one device share it, so issue them on

@@ -51,6 +51,7 @@ struct Args {
   double h2;
   int bilinear, any;
   int rows, strips_x, items;
+  const int* done;        // solver's flag (null: none): nothing to do where it is set
 };
 
 // Inputs of one row step (read back as 16-byte pairs, so its size is a multiple of 16).
@@ -298,8 +299,11 @@ template <int NU, bool DOWN, bool PRO>
 __global__ void __launch_bounds__(32 * kWarps, NU < 3 ? 4 : 3) emb_strip_kernel(const __grid_constant__ Args A) {
   __shared__ __align__(16) Step<PRO> ring[kWarps][kRing];
   constexpr int T = 2 * NU;
+  tma::pdl_trigger();
   const int warp = threadIdx.x >> 5, item = blockIdx.x * kWarps + warp;
   if (item >= A.items) return;
+  tma::pdl_wait();
+  if (A.done && *A.done) return;
   const int tj = item / A.strips_x, ti = item - tj * A.strips_x;
   const int x0 = ti * 2 * lanes(NU, DOWN) - 2 * lo(NU, DOWN), r0 = tj * A.rows;
   // rows read: down to r0 - T - 2 and up to r0 + rows + T + 7 (the last unrolled step runs over)

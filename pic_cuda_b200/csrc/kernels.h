@@ -155,6 +155,7 @@ struct EmbLevels {
   uint8_t* mask[PIC_MAX_LEVELS] = {};
   const double* bc[PIC_MAX_LEVELS] = {};
   double h = 0.0;
+  const int* done = nullptr;   // device flag: the V-cycle's kernels return at once where it is set
 };
 // Level sizes and the first level the one-CTA kernel solves.
 void emb_layout(EmbLevels& P, int nx, int ny, int levels);

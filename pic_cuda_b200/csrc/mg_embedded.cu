@@ -35,7 +35,13 @@
 //   emb_coarse_kernel  every level from the first one with at most 65 x 65 nodes down, in one
 //       CTA's shared memory (one launch for the whole lower V-cycle).
 //   emb_norm_kernel / emb_norm_final_kernel  ||r||^2 and ||rhs||^2 over the FLUID nodes in a
-//       fixed order (per-CTA partials, then one CTA), for the convergence test.
+//       fixed order (per-CTA partials, then one CTA), for the convergence test, which the last of
+//       them makes: it sets the solve's done flag, and the host sends cycles in groups instead of
+//       waiting for each one's norm (385 x 257, 50 cycles: 4.78 -> 3.69 ms, the wait, the copy and
+//       the restart having taken 20 us of a cycle's 97).
+// At 385 x 257 a V-cycle is a chain of eleven short launches (10 us or less each but for the coarse
+// kernel's 21); programmatic launches let each one's start-up overlap its predecessor's end
+// (77.8 -> 76.4 us a V-cycle; 1025^2 133.8 -> 123.4).
 // The shared tiles store each colour's nodes contiguously (struct Tile), so a red-black
 // half-sweep reads its FP64 neighbours at unit stride.
 #include <algorithm>
@@ -189,14 +195,23 @@ __device__ __forceinline__ void store_tile(const Tile<W>& T, double* __restrict_
   }
 }
 
+// Start of every kernel of a solve: the next launch may begin its own start-up, this one waits for the
+// previous one's results, and where the solver's flag is set there is nothing left to do.
+__device__ __forceinline__ bool skip_launch(const int* done) {
+  tma::pdl_trigger();
+  tma::pdl_wait();
+  return done && *done;
+}
+
 // NU sweeps (post-smoothing with PRO: after adding the coarse correction) of one tile.
 template <int NU, bool PRO>
 __global__ void __launch_bounds__(kSmoothThreads) emb_smooth_kernel(
     const double* __restrict__ phi_in, double* __restrict__ phi_out, const double* __restrict__ rhs,
     const uint8_t* __restrict__ mask, const double* __restrict__ bc, const double* __restrict__ coarse, int nx, int ny,
-    int nxc, double h2, int bilinear) {
+    int nxc, double h2, int bilinear, const int* done) {
   constexpr int H = 2 * NU, W = kTile + 2 * H;
   __shared__ Tile<W> T;
+  if (skip_launch(done)) return;
   const int x0 = blockIdx.x * kTile - H, y0 = blockIdx.y * kTile - H;
   stage_tile<W, PRO>(T, phi_in, rhs, mask, bc, coarse, nx, ny, nxc, x0, y0, bilinear != 0);
   __syncthreads();
@@ -245,9 +260,11 @@ template <int NU>
 __global__ void __launch_bounds__(kSmoothThreads) emb_down_kernel(
     const double* __restrict__ phi_in, double* __restrict__ phi_out, const double* __restrict__ rhs,
     const uint8_t* __restrict__ mask, const double* __restrict__ bc, int nx, int ny, double h2,
-    double* __restrict__ rhs_c, uint8_t* __restrict__ mask_c, double* __restrict__ phi_c, int nxc, int nyc, int any) {
+    double* __restrict__ rhs_c, uint8_t* __restrict__ mask_c, double* __restrict__ phi_c, int nxc, int nyc, int any,
+    const int* done) {
   constexpr int H = 2 * NU + 2, W = kTile + 2 * H;
   __shared__ Tile<W> T;
+  if (skip_launch(done)) return;
   const int x0 = blockIdx.x * kTile - H, y0 = blockIdx.y * kTile - H;
   stage_tile<W, false>(T, phi_in, rhs, mask, bc, nullptr, nx, ny, 0, x0, y0, false);
   __syncthreads();
@@ -293,30 +310,32 @@ struct CoarseLevelArgs {
   double h2[PIC_MAX_LEVELS];
   int soff[PIC_MAX_LEVELS];  // byte offsets in shared memory: phi, rb (doubles), then kinds
   int nu1, nu2, coarsen_any, bilinear;
+  const int* done;
 };
 
+// The lower levels in one CTA: a warp takes a row, its lanes the row's nodes (of one colour in a
+// half-sweep), so no thread divides by the row length.  Bound by the latency of the chain of
+// half-sweeps, barriers and FP64 divisions on one SM (65 x 65 and below, 2 + 2 sweeps: 24 -> 21 us
+// against a flat index over the level).
 __device__ void cta_half_sweep(double* p, const double* rb, const uint8_t* m, int nx, int ny, int colour, double h2) {
-  const int half = (nx - 1) / 2;            // >= nodes of one colour per interior row
-  const int cnt = (ny - 2) * half;
-  for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
-    const int r = k / half;
-    const int j = 1 + r;
-    const int i = 1 + ((1 + j + colour) & 1) + 2 * (k - r * half);
-    if (i >= nx - 1) continue;
-    const int t = j * nx + i;
-    const uint8_t kk = m[t];
-    if (kk == kFluid) {
-      const double sum = p[t - nx] + p[t + nx] + p[t - 1] + p[t + 1];
-      p[t] = 0.25 * (sum - h2 * rb[t]);
-    } else if (kk == kDir) {
-      p[t] = rb[t];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  for (int j = 1 + warp; j < ny - 1; j += nwarp)
+    for (int i = 1 + ((1 + j + colour) & 1) + 2 * lane; i < nx - 1; i += 64) {
+      const int t = j * nx + i;
+      const uint8_t kk = m[t];
+      if (kk == kFluid) {
+        const double sum = p[t - nx] + p[t + nx] + p[t - 1] + p[t + 1];
+        p[t] = 0.25 * (sum - h2 * rb[t]);
+      } else if (kk == kDir) {
+        p[t] = rb[t];
+      }
     }
-  }
 }
 
 __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int T = blockDim.x;
+  if (skip_launch(A.done)) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   auto P = [&](int l) { return reinterpret_cast<double*>(smem + A.soff[l]); };
   auto RB = [&](int l) { return reinterpret_cast<double*>(smem + A.soff[l]) + A.nx[l] * A.ny[l]; };
   auto M = [&](int l) { return reinterpret_cast<uint8_t*>(smem + A.soff[l] + 16 * A.nx[l] * A.ny[l]); };
@@ -324,17 +343,19 @@ __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelA
   {
     const int nx = A.nx[0], ny = A.ny[0];
     double* p = P(0); double* rb = RB(0); uint8_t* m = M(0);
-    for (int k = threadIdx.x; k < nx * ny; k += T) {
-      const int j = k / nx, i = k - j * nx;
-      p[k] = A.phi[0][k];
-      uint8_t kk = kFixed;
-      double v = 0.0;
-      if (i > 0 && j > 0 && i < nx - 1 && j < ny - 1) {
-        kk = smoother_kind(A.mask[0][k], A.bc[0] != nullptr);
-        v = kk == kFluid ? A.rhs[0][k] : kk == kDir ? A.bc[0][k] : 0.0;
+#pragma unroll 4
+    for (int j = warp; j < ny; j += nwarp)
+      for (int i = lane; i < nx; i += 32) {
+        const int k = j * nx + i;
+        p[k] = A.phi[0][k];
+        uint8_t kk = kFixed;
+        double v = 0.0;
+        if (i > 0 && j > 0 && i < nx - 1 && j < ny - 1) {
+          kk = smoother_kind(A.mask[0][k], A.bc[0] != nullptr);
+          v = kk == kFluid ? A.rhs[0][k] : kk == kDir ? A.bc[0][k] : 0.0;
+        }
+        m[k] = kk; rb[k] = v;
       }
-      m[k] = kk; rb[k] = v;
-    }
   }
   __syncthreads();
   // down leg
@@ -355,29 +376,33 @@ __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelA
     const uint8_t* mk = A.mask[l];   // reference kinds of level l (written above for l > 0)
     const double h2i = 1.0 / A.h2[l];
     double* pc = P(l + 1); double* rbc = RB(l + 1); uint8_t* mc = M(l + 1);
-    for (int k = threadIdx.x; k < nxc * nyc; k += T) {
-      const int jc = k / nxc, ic = k - jc * nxc;
-      pc[k] = 0.0;
-      uint8_t kc = kFluid;
-      double fc = 0.0;
-      if (ic > 0 && jc > 0 && ic < nxc - 1 && jc < nyc - 1) {
-        const ptrdiff_t idf = (ptrdiff_t)(2 * jc) * nx + 2 * ic;
-        kc = coarse_kind_of([&](int di, int dj) { return mk[idf + (ptrdiff_t)dj * nx + di]; }, A.coarsen_any != 0);
-        if (kc == kFluid)
-          fc = full_weight([&](int di, int dj) {
-                 const ptrdiff_t id = idf + (ptrdiff_t)dj * nx + di;
-                 if (mk[id] != kFluid) return 0.0;
-                 const double lap = pf[id - nx] + pf[id + nx] + pf[id - 1] + pf[id + 1] - 4.0 * pf[id];
-                 return rbf[id] - h2i * lap;
-               });
+    for (int jc = warp; jc < nyc; jc += nwarp)
+      for (int ic = lane; ic < nxc; ic += 32) {
+        const int k = jc * nxc + ic;
+        pc[k] = 0.0;
+        uint8_t kc = kFluid;
+        double fc = 0.0;
+        const bool interior = ic > 0 && jc > 0 && ic < nxc - 1 && jc < nyc - 1;
+        if (interior) {
+          const int idf = 2 * jc * nx + 2 * ic;
+          uint8_t kind[9];
+#pragma unroll
+          for (int q = 0; q < 9; ++q) kind[q] = mk[idf + (q / 3 - 1) * nx + (q % 3 - 1)];
+          kc = coarse_kind_of([&](int di, int dj) { return kind[(dj + 1) * 3 + di + 1]; }, A.coarsen_any != 0);
+          if (kc == kFluid)
+            fc = full_weight([&](int di, int dj) {
+                   const int id = idf + dj * nx + di;
+                   if (kind[(dj + 1) * 3 + di + 1] != kFluid) return 0.0;
+                   const double lap = pf[id - nx] + pf[id + nx] + pf[id - 1] + pf[id + 1] - 4.0 * pf[id];
+                   return rbf[id] - h2i * lap;
+                 });
+        }
+        A.mask[l + 1][k] = kc;       // the reference writes the coarse kinds and rhs of every level
+        A.rhs[l + 1][k] = fc;
+        const uint8_t sk = interior ? smoother_kind(kc, A.bc[l + 1] != nullptr) : kFixed;
+        mc[k] = sk;
+        rbc[k] = sk == kFluid ? fc : sk == kDir ? A.bc[l + 1][k] : 0.0;
       }
-      A.mask[l + 1][k] = kc;       // the reference writes the coarse kinds and rhs of every level
-      A.rhs[l + 1][k] = fc;
-      const bool interior = ic > 0 && jc > 0 && ic < nxc - 1 && jc < nyc - 1;
-      const uint8_t sk = interior ? smoother_kind(kc, A.bc[l + 1] != nullptr) : kFixed;
-      mc[k] = sk;
-      rbc[k] = sk == kFluid ? fc : sk == kDir ? A.bc[l + 1][k] : 0.0;
-    }
     __syncthreads();
   }
   // up leg
@@ -386,11 +411,11 @@ __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelA
     double* p = P(l);
     const double* pc = P(l + 1);
     const uint8_t* m = M(l);
-    for (int k = threadIdx.x; k < nx * ny; k += T) {
-      const int j = k / nx, i = k - j * nx;
-      const bool interior = i > 0 && j > 0 && i < nx - 1 && j < ny - 1;
-      if (interior && m[k] == kFluid) p[k] += prolong_at(pc, nxc, i, j, A.bilinear != 0);
-    }
+    for (int j = 1 + warp; j < ny - 1; j += nwarp)
+      for (int i = 1 + lane; i < nx - 1; i += 32) {
+        const int k = j * nx + i;
+        if (m[k] == kFluid) p[k] += prolong_at(pc, nxc, i, j, A.bilinear != 0);
+      }
     __syncthreads();
     for (int s = 0; s < 2 * A.nu2; ++s) {
       cta_half_sweep(p, RB(l), m, nx, ny, s & 1, A.h2[l]);
@@ -401,7 +426,7 @@ __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelA
   for (l = 0; l < A.n; ++l) {
     const int N = A.nx[l] * A.ny[l];
     const double* p = P(l);
-    for (int k = threadIdx.x; k < N; k += T) A.phi[l][k] = p[k];
+    for (int k = threadIdx.x; k < N; k += blockDim.x) A.phi[l][k] = p[k];
   }
 }
 
@@ -422,8 +447,9 @@ __device__ double cta_sum(double v, double* red) {
 // partial is formed in a fixed order.
 __global__ void __launch_bounds__(256) emb_norm_kernel(const double* __restrict__ phi, const double* __restrict__ rhs,
                                                        const uint8_t* __restrict__ mask, int nx, int ny, double h2i,
-                                                       double* __restrict__ partials) {
+                                                       double* __restrict__ partials, const int* done) {
   __shared__ double red[8];
+  if (skip_launch(done)) return;
   double r2 = 0.0, f2 = 0.0;
   for (int j = 1 + blockIdx.x; j < ny - 1; j += gridDim.x) {
     const size_t row = (size_t)j * nx;
@@ -440,14 +466,41 @@ __global__ void __launch_bounds__(256) emb_norm_kernel(const double* __restrict_
   if (threadIdx.x == 0) { partials[2 * blockIdx.x] = a; partials[2 * blockIdx.x + 1] = b; }
 }
 
+// What a solve knows of itself, on the device and (copied) on the host.
+struct SolveState {
+  double r2, f2;       // ||r||^2 and ||rhs||^2 of the last norms
+  double r0;           // ||r||^2 of the initial guess
+  double rel, before;  // relative residual of the last check, and of the one before
+  int cycles, done;
+};
+
+__device__ __forceinline__ double emb_relative(double r2, double f2, double r0) {
+  if (f2 > 0.0) return sqrt(r2 / f2);
+  if (r0 > 0.0) return sqrt(r2 / r0);
+  return sqrt(r2);
+}
+
+// The norms from the partials in a fixed order.  cycle >= 0: they belong to a V-cycle of the solve, which
+// is counted and ends the solve below tol; -1: to the initial guess.
 __global__ void __launch_bounds__(256) emb_norm_final_kernel(const double* __restrict__ partials, int n,
-                                                             double* __restrict__ out) {
+                                                             SolveState* __restrict__ S, int cycle, double tol,
+                                                             const int* done) {
   __shared__ double red[8];
+  if (skip_launch(done)) return;
   double a = 0.0, b = 0.0;
   for (int k = threadIdx.x; k < n; k += 256) { a += partials[2 * k]; b += partials[2 * k + 1]; }
   a = cta_sum(a, red);
   b = cta_sum(b, red);
-  if (threadIdx.x == 0) { out[0] = a; out[1] = b; }
+  if (threadIdx.x == 0) {
+    S->r2 = a; S->f2 = b;
+    if (cycle < 0) { S->r0 = a; S->cycles = 0; S->done = 0; }
+    S->before = S->rel;
+    S->rel = emb_relative(a, b, S->r0);
+    if (cycle >= 0) {
+      S->cycles = cycle + 1;
+      if (S->rel < tol) S->done = 1;
+    }
+  }
 }
 
 }  // namespace
@@ -479,6 +532,23 @@ int coarse_smem_bytes(const EmbLevels& P, int l0, int offs[PIC_MAX_LEVELS]) {
   return off;
 }
 
+// Launch with programmatic stream serialisation (every kernel here waits in skip_launch or pdl_wait before
+// it reads its predecessor's results).
+template <typename... KArgs, typename... Args>
+void launch_emb(void (*k)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 // Arguments of the strip kernels (emb_strips.cuh) for nu sweeps of a level (down: with the
 // restriction); rows = 0 where the tile kernels take it.  An item is one warp with FP64 chains to hide, so
 // a level needs about 14 of them per SM; the largest row count that still gives as many wastes
@@ -496,6 +566,7 @@ embs::Args strip_args(const EmbLevels& P, int l, int nu, bool down, const double
     cudaGetLastError();
     return A;
   }
+  A.done = P.done;
   A.phi = in; A.out = out; A.rhs = P.rhs[l]; A.mask = P.mask[l]; A.bc = P.bc[l];
   A.nx = nx; A.ny = ny;
   A.h2 = P.h * P.h * std::ldexp(1.0, 2 * l);
@@ -516,14 +587,15 @@ void launch_smooth(const EmbLevels& P, int l, const double* in, double* out, con
       A.coarse = coarse;
       A.bilinear = bilinear ? 1 : 0;
       if (PRO) { A.nxc = P.nx[l + 1]; A.nyc = P.ny[l + 1]; }
-      embs::emb_strip_kernel<NU, false, PRO><<<(A.items + embs::kWarps - 1) / embs::kWarps, 32 * embs::kWarps, 0, s>>>(A);
+      launch_emb(embs::emb_strip_kernel<NU, false, PRO>, dim3((A.items + embs::kWarps - 1) / embs::kWarps), 32 * embs::kWarps, 0, s,
+                 A);
       return;
     }
   }
   const dim3 grid((P.nx[l] + kTile - 1) / kTile, (P.ny[l] + kTile - 1) / kTile);
   const double h2 = P.h * P.h * std::ldexp(1.0, 2 * l);
-  emb_smooth_kernel<NU, PRO><<<grid, kSmoothThreads, 0, s>>>(in, out, P.rhs[l], P.mask[l], P.bc[l], coarse, P.nx[l],
-                                                            P.ny[l], PRO ? P.nx[l + 1] : 0, h2, bilinear ? 1 : 0);
+  launch_emb(emb_smooth_kernel<NU, PRO>, grid, kSmoothThreads, 0, s, in, out, (const double*)P.rhs[l],
+             (const uint8_t*)P.mask[l], P.bc[l], coarse, P.nx[l], P.ny[l], PRO ? P.nx[l + 1] : 0, h2, bilinear ? 1 : 0, P.done);
 }
 
 void smooth_chunk(const EmbLevels& P, int l, int nu, bool pro, const double* in, double* out, bool bilinear,
@@ -551,15 +623,15 @@ void launch_down(const EmbLevels& P, int l, const double* in, double* out, int a
       A.nxc = P.nx[l + 1]; A.nyc = P.ny[l + 1];
       A.rhs_c = P.rhs[l + 1]; A.mask_c = P.mask[l + 1]; A.phi_c = P.phi[l + 1];
       A.any = any;
-      embs::emb_strip_kernel<NU, true, false><<<(A.items + embs::kWarps - 1) / embs::kWarps, 32 * embs::kWarps, 0, s>>>(A);
+      launch_emb(embs::emb_strip_kernel<NU, true, false>, dim3((A.items + embs::kWarps - 1) / embs::kWarps), 32 * embs::kWarps, 0, s,
+                 A);
       return;
     }
   }
   const dim3 grid((P.nx[l] + kTile - 1) / kTile, (P.ny[l] + kTile - 1) / kTile);
   const double h2 = P.h * P.h * std::ldexp(1.0, 2 * l);
-  emb_down_kernel<NU><<<grid, kSmoothThreads, 0, s>>>(in, out, P.rhs[l], P.mask[l], P.bc[l], P.nx[l], P.ny[l], h2,
-                                                     P.rhs[l + 1], P.mask[l + 1], P.phi[l + 1], P.nx[l + 1],
-                                                     P.ny[l + 1], any);
+  launch_emb(emb_down_kernel<NU>, grid, kSmoothThreads, 0, s, in, out, (const double*)P.rhs[l], (const uint8_t*)P.mask[l],
+             P.bc[l], P.nx[l], P.ny[l], h2, P.rhs[l + 1], P.mask[l + 1], P.phi[l + 1], P.nx[l + 1], P.ny[l + 1], any, P.done);
 }
 
 // nu sweeps of level l (chunks of at most 4 per launch; the first applies the prolongation
@@ -631,7 +703,8 @@ int emb_vcycle(const EmbLevels& P, int l0, int nu1, int nu2, int options, cudaSt
     }
     const int bytes = coarse_smem_bytes(P, lc, A.soff);
     A.nu1 = nu1; A.nu2 = nu2; A.coarsen_any = any; A.bilinear = bilinear ? 1 : 0;
-    emb_coarse_kernel<<<1, kCoarseThreads, bytes, s>>>(A);
+    A.done = P.done;
+    launch_emb(emb_coarse_kernel, dim3(1), kCoarseThreads, bytes, s, A);
   }
   for (int l = std::min(lc, P.L - 1) - 1; l >= l0; --l) {
     smooth_level(P, l, nu2, true, cur[l], bilinear, s);
@@ -645,16 +718,21 @@ int emb_vcycle(const EmbLevels& P, int l0, int nu1, int nu2, int options, cudaSt
   return PIC_OK;
 }
 
-// ||r||^2 and ||rhs||^2 over level 0's FLUID nodes into out (device, 2 doubles).
-int emb_norms(const EmbLevels& P, double* partials, double* out, cudaStream_t s) {
+namespace {
+
+// ||r||^2 and ||rhs||^2 over level 0's FLUID nodes into S; see emb_norm_final_kernel.
+int emb_norms(const EmbLevels& P, double* partials, SolveState* S, int cycle, double tol, cudaStream_t s) {
   const double h2i = 1.0 / (P.h * P.h);
   const int nb = std::max(1, std::min(kNormBlocks, P.ny[0] - 2));
-  emb_norm_kernel<<<nb, 256, 0, s>>>(P.phi[0], P.rhs[0], P.mask[0], P.nx[0], P.ny[0], h2i, partials);
-  emb_norm_final_kernel<<<1, 256, 0, s>>>(partials, nb, out);
+  launch_emb(emb_norm_kernel, dim3(nb), 256, 0, s, (const double*)P.phi[0], (const double*)P.rhs[0],
+             (const uint8_t*)P.mask[0], P.nx[0], P.ny[0], h2i, partials, P.done);
+  launch_emb(emb_norm_final_kernel, dim3(1), 256, 0, s, (const double*)partials, nb, S, cycle, tol, P.done);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return pic_fail(PIC_ERR_CUDA, cudaGetErrorString(e));
   return PIC_OK;
 }
+
+}  // namespace
 
 namespace {
 
@@ -665,8 +743,8 @@ struct EmbScratch {
   EmbLevels P;           // coarse-level pointers (level 0 is filled per call)
   double* alt0;
   double* partials;
-  double* norms;         // device, 2 doubles
-  double* host_norms;    // pinned, 2 doubles
+  SolveState* state;       // device
+  SolveState* host_state;  // pinned
 };
 std::mutex g_emb_mu;
 std::vector<EmbScratch> g_emb;
@@ -692,9 +770,9 @@ int emb_scratch(int device, int nx, int ny, int levels, EmbScratch** out) {
     if (e == cudaSuccess) e = A((void**)&c.P.mask[l], N);
   }
   if (e == cudaSuccess) e = A((void**)&c.partials, sizeof(double) * 2 * kNormBlocks);
-  if (e == cudaSuccess) e = A((void**)&c.norms, sizeof(double) * 2);
+  if (e == cudaSuccess) e = A((void**)&c.state, sizeof(SolveState));
   if (e == cudaSuccess) {
-    e = cudaMallocHost((void**)&c.host_norms, sizeof(double) * 2);
+    e = cudaMallocHost((void**)&c.host_state, sizeof(SolveState));
   }
   if (e != cudaSuccess) {
     for (void* p : got) cudaFree(p);
@@ -706,10 +784,14 @@ int emb_scratch(int device, int nx, int ny, int levels, EmbScratch** out) {
   return PIC_OK;
 }
 
-double emb_relative(const double n[2], double r0) {
-  if (n[1] > 0.0) return std::sqrt(n[0] / n[1]);
-  if (r0 > 0.0) return std::sqrt(n[0] / r0);
-  return std::sqrt(n[0]);
+// V-cycles to send before the next look at the norms: one fewer than the last two residuals' ratio says
+// are needed (the kernels of cycles behind the converged one return at once, but each still costs its
+// launches).
+int cycles_ahead(const SolveState& S, double tol, int left) {
+  int n = 1;
+  if (S.cycles >= 2 && S.rel > tol && S.rel < S.before && S.rel > 0.0)
+    n = (int)std::min(16.0, std::ceil(std::log(tol / S.rel) / std::log(S.rel / S.before))) - 1;
+  return std::max(1, std::min(n, left));
 }
 
 }  // namespace
@@ -736,35 +818,42 @@ extern "C" int pic_solve_embedded_f64(double* phi, const double* rhs, const uint
   P.phi[0] = phi; P.alt[0] = S->alt0; P.rhs[0] = const_cast<double*>(rhs);
   P.mask[0] = const_cast<uint8_t*>(mask); P.bc[0] = phi_bc; P.h = h;
   cudaStream_t s = (cudaStream_t)stream;
+  // With a tolerance the norms follow every cycle on the device, where the first cycle below tol sets the
+  // done flag, and the host sends several cycles at a time.  The kernels of a cycle behind the converged
+  // one return at once; its cudaMemcpyAsync copies (an odd number of smoothing launches per level) repeat
+  // the converged cycle's copies from arrays that nothing has written since.
   const bool check = tol > 0;
-  double r0 = 0.0, n[2] = {0.0, 0.0};
-  auto read_norms = [&]() -> int {
-    int r = emb_norms(P, S->partials, S->norms, s);
-    if (r) return r;
-    cudaError_t e2 = cudaMemcpyAsync(S->host_norms, S->norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
+  auto read_state = [&]() -> int {
+    cudaError_t e2 = cudaMemcpyAsync(S->host_state, S->state, sizeof(SolveState), cudaMemcpyDeviceToHost, s);
     if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(s);
-    if (e2 != cudaSuccess) return pic_fail(PIC_ERR_CUDA, cudaGetErrorString(e2));
-    n[0] = S->host_norms[0]; n[1] = S->host_norms[1];
-    return PIC_OK;
+    return e2 == cudaSuccess ? PIC_OK : pic_fail(PIC_ERR_CUDA, cudaGetErrorString(e2));
   };
-  if (check || relres_out) {
-    if ((rc = read_norms())) return rc;
-    r0 = n[0];
-  }
   int cyc = 0;
-  double rel = emb_relative(n, r0);
-  while (cyc < max_cycles) {
-    if ((rc = emb_vcycle(P, 0, nu_pre, nu_post, options, s))) return rc;
-    ++cyc;
-    if (check) {
-      if ((rc = read_norms())) return rc;
-      rel = emb_relative(n, r0);
-      if (rel < tol) break;
-    }
+  double rel = 0.0;
+  if (check || relres_out) {
+    if ((rc = emb_norms(P, S->partials, S->state, -1, tol, s))) return rc;
   }
-  if (!check && relres_out) {
-    if ((rc = read_norms())) return rc;
-    rel = emb_relative(n, r0);
+  if (check) {
+    P.done = &S->state->done;
+    for (int ahead = std::min(2, max_cycles);;) {
+      for (int k = 0; k < ahead; ++k) {
+        if ((rc = emb_vcycle(P, 0, nu_pre, nu_post, options, s))) return rc;
+        if ((rc = emb_norms(P, S->partials, S->state, cyc + k, tol, s))) return rc;
+      }
+      if ((rc = read_state())) return rc;
+      cyc = S->host_state->cycles;
+      rel = S->host_state->rel;
+      if (S->host_state->done || cyc >= max_cycles) break;
+      ahead = cycles_ahead(*S->host_state, tol, max_cycles - cyc);
+    }
+  } else {
+    for (; cyc < max_cycles; ++cyc)
+      if ((rc = emb_vcycle(P, 0, nu_pre, nu_post, options, s))) return rc;
+    if (relres_out) {
+      if ((rc = emb_norms(P, S->partials, S->state, max_cycles - 1, 0.0, s))) return rc;
+      if ((rc = read_state())) return rc;
+      rel = S->host_state->rel;
+    }
   }
   if (cycles_out) *cycles_out = cyc;
   if (relres_out) *relres_out = rel;
