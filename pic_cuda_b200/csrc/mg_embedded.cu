@@ -34,14 +34,15 @@
 //       (emb_strip_kernel, emb_strips.cuh), with the same bits.
 //   emb_coarse_kernel  every level from the first one with at most 65 x 65 nodes down, in one
 //       CTA's shared memory (one launch for the whole lower V-cycle).
-//   emb_norm_kernel / emb_norm_final_kernel  ||r||^2 and ||rhs||^2 over the FLUID nodes in a
-//       fixed order (per-CTA partials, then one CTA), for the convergence test, which the last of
-//       them makes: it sets the solve's done flag, and the host sends cycles in groups instead of
+//   emb_norm_kernel  ||r||^2 and ||rhs||^2 over the FLUID nodes in a fixed order (per-CTA
+//       partials, then the last CTA), for the convergence test, which that CTA makes: it sets the solve's done flag, and the host sends cycles in groups instead of
 //       waiting for each one's norm (385 x 257, 50 cycles: 4.78 -> 3.69 ms, the wait, the copy and
 //       the restart having taken 20 us of a cycle's 97).
-// At 385 x 257 a V-cycle is a chain of eleven short launches (10 us or less each but for the coarse
-// kernel's 21); programmatic launches let each one's start-up overlap its predecessor's end
-// (77.8 -> 76.4 us a V-cycle; 1025^2 133.8 -> 123.4).
+// At 385 x 257 a cycle is a chain of eight short launches, each bound by its own chain of loads,
+// half-sweeps and barriers, not by bandwidth: programmatic launches overlap each one's start-up with its
+// predecessor's end (V-cycle 77.8 -> 76.4 us; 1025^2 133.8 -> 123.4), and a CTA of 1024 threads, one node
+// of each colour per thread, shortens the chain (76 -> 54 us; 1025^2 124 -> 103; with 256 threads on
+// 16 x 16 tiles 61 and 127); with the one-CTA kernel's share 48 and 95 us.
 // The shared tiles store each colour's nodes contiguously (struct Tile), so a red-black
 // half-sweep reads its FP64 neighbours at unit stride.
 #include <algorithm>
@@ -61,8 +62,8 @@ namespace {
 constexpr uint8_t kFluid = PIC_NODE_FLUID, kDir = PIC_NODE_DIRICHLET, kSolid = PIC_NODE_SOLID;
 constexpr uint8_t kFixed = 255;            // grid boundary / outside the grid: never updated
 constexpr int kTile = 32;
-constexpr int kSmoothThreads = 256;
-constexpr int kCoarseThreads = 512;
+constexpr int kSmoothThreads = 1024;
+constexpr int kCoarseThreads = 1024;
 constexpr int kCoarseMaxNodes = 65 * 65;   // first level at or below this size: one-CTA solve
 constexpr int kNormBlocks = 592;
 
@@ -112,28 +113,50 @@ struct Tile {
   }
 };
 
-// One colour of smooth_redblack on the interior tile nodes: thread k takes row 1 + k / H and
-// the k-th node of that colour in it (H = (W-2)/2 per row), so no thread skips nodes.  FLUID
-// nodes relax, DIRICHLET nodes take their phi_bc when the caller gave one, others stay.
-template <int W>
-__device__ __forceinline__ void tile_half_sweep(Tile<W>& T, int colour, double h2, bool has_bc) {
+// NU sweeps of smooth_redblack on the interior tile nodes, colour (i + j) even first.  Thread k has one
+// node of each colour, the (k % H)-th one of its colour in row 1 + k / H (H = (W - 2) / 2 per row), and a
+// second pair 1024 nodes further on where the tile is that large (four sweeps): their kinds and right-hand sides stay in registers, and a half-sweep is four
+// shared loads, the FP64 chain and a barrier.  FLUID nodes relax, DIRICHLET nodes take their phi_bc when
+// the caller gave one, others stay.
+template <int W, int NU>
+__device__ __forceinline__ void tile_sweeps(Tile<W>& T, double h2, bool has_bc) {
+  if (NU == 0) return;
   constexpr int HW = W / 2, HALF = (W - 2) / 2, CNT = (W - 2) * HALF;
-  double* __restrict__ own = T.p[colour];
-  const double* __restrict__ oth = T.p[colour ^ 1];
-  const double* __restrict__ rb = T.rb[colour];
-  const uint8_t* __restrict__ mk = T.m[colour];
-  for (int k = threadIdx.x; k < CNT; k += kSmoothThreads) {
-    const int r = k / HALF;
-    const int ty = 1 + r;
-    const int odd = (colour - ty) & 1;              // tx parity of this colour in row ty
-    const int i = ty * HW + (k - r * HALF) + (odd ? 0 : 1);
-    const uint8_t m = mk[i];
-    if (m == kFluid) {
-      const int w = i - 1 + odd;
-      const double sum = oth[i - HW] + oth[i + HW] + oth[w] + oth[w + 1];
-      own[i] = 0.25 * (sum - h2 * rb[i]);
-    } else if (m == kDir && has_bc) {
-      own[i] = rb[i];
+  constexpr int IT = (CNT + kSmoothThreads - 1) / kSmoothThreads;
+  int at[IT], par[IT];
+  double rb[IT][2];
+  uint8_t m[IT][2];
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int k = threadIdx.x + it * kSmoothThreads;
+    const int r = k / HALF, ty = 1 + r;
+    const int base = ty * HW + (k - r * HALF);
+    at[it] = base;
+    par[it] = ty & 1;        // tx parity of colour 0 in row ty
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int i = base + ((par[it] ^ c) ? 0 : 1);
+      m[it][c] = kFixed; rb[it][c] = 0.0;
+      if (k < CNT) { m[it][c] = T.m[c][i]; rb[it][c] = T.rb[c][i]; }
+    }
+  }
+#pragma unroll 1
+  for (int s = 0; s < NU; ++s) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      double* __restrict__ own = T.p[c];
+      const double* __restrict__ oth = T.p[c ^ 1];
+#pragma unroll
+      for (int it = 0; it < IT; ++it) {
+        const int odd = par[it] ^ c, i = at[it] + 1 - odd;
+        if (m[it][c] == kFluid) {
+          const double sum = oth[i - HW] + oth[i + HW] + oth[at[it]] + oth[at[it] + 1];
+          own[i] = 0.25 * fma(-h2, rb[it][c], sum);   // written out: h2 * rb must not be kept as a product
+        } else if (m[it][c] == kDir && has_bc) {
+          own[i] = rb[it][c];
+        }
+      }
+      __syncthreads();
     }
   }
 }
@@ -215,11 +238,7 @@ __global__ void __launch_bounds__(kSmoothThreads) emb_smooth_kernel(
   const int x0 = blockIdx.x * kTile - H, y0 = blockIdx.y * kTile - H;
   stage_tile<W, PRO>(T, phi_in, rhs, mask, bc, coarse, nx, ny, nxc, x0, y0, bilinear != 0);
   __syncthreads();
-#pragma unroll 1
-  for (int s = 0; s < 2 * NU; ++s) {
-    tile_half_sweep<W>(T, s & 1, h2, bc != nullptr);
-    __syncthreads();
-  }
+  tile_sweeps<W, NU>(T, h2, bc != nullptr);
   store_tile<W, H>(T, phi_out, nx, ny, x0, y0);
 }
 
@@ -268,16 +287,13 @@ __global__ void __launch_bounds__(kSmoothThreads) emb_down_kernel(
   const int x0 = blockIdx.x * kTile - H, y0 = blockIdx.y * kTile - H;
   stage_tile<W, false>(T, phi_in, rhs, mask, bc, nullptr, nx, ny, 0, x0, y0, false);
   __syncthreads();
-#pragma unroll 1
-  for (int s = 0; s < 2 * NU; ++s) {
-    tile_half_sweep<W>(T, s & 1, h2, bc != nullptr);
-    __syncthreads();
-  }
+  tile_sweeps<W, NU>(T, h2, bc != nullptr);
   store_tile<W, H>(T, phi_out, nx, ny, x0, y0);
   const double h2i = 1.0 / h2;
-  const int k = threadIdx.x;            // 256 threads, one coarse node each
-  const int ic = blockIdx.x * (kTile / 2) + (k & 15), jc = blockIdx.y * (kTile / 2) + (k >> 4);
-  if (ic >= nxc || jc >= nyc) return;
+  constexpr int CT = kTile / 2;
+  const int k = threadIdx.x;            // one coarse node each
+  const int ic = blockIdx.x * CT + k % CT, jc = blockIdx.y * CT + k / CT;
+  if (k >= CT * CT || ic >= nxc || jc >= nyc) return;
   const size_t idc = (size_t)jc * nxc + ic;
   phi_c[idc] = 0.0;
   if (ic == 0 || jc == 0 || ic == nxc - 1 || jc == nyc - 1) {
@@ -307,31 +323,67 @@ struct CoarseLevelArgs {
   double* rhs[PIC_MAX_LEVELS];
   uint8_t* mask[PIC_MAX_LEVELS];
   const double* bc[PIC_MAX_LEVELS];
-  double h2[PIC_MAX_LEVELS];
-  int soff[PIC_MAX_LEVELS];  // byte offsets in shared memory: phi, rb (doubles), then kinds
+  double h2[PIC_MAX_LEVELS], h2i[PIC_MAX_LEVELS];
+  int soff[PIC_MAX_LEVELS];  // byte offsets in shared memory: phi, rb (doubles), then both kinds
   int nu1, nu2, coarsen_any, bilinear;
   const int* done;
 };
 
-// The lower levels in one CTA: a warp takes a row, its lanes the row's nodes (of one colour in a
-// half-sweep), so no thread divides by the row length.  Bound by the latency of the chain of
-// half-sweeps, barriers and FP64 divisions on one SM (65 x 65 and below, 2 + 2 sweeps: 24 -> 21 us
-// against a flat index over the level).
-__device__ void cta_half_sweep(double* p, const double* rb, const uint8_t* m, int nx, int ny, int colour, double h2) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  for (int j = 1 + warp; j < ny - 1; j += nwarp)
-    for (int i = 1 + ((1 + j + colour) & 1) + 2 * lane; i < nx - 1; i += 64) {
-      const int t = j * nx + i;
-      const uint8_t kk = m[t];
-      if (kk == kFluid) {
-        const double sum = p[t - nx] + p[t + nx] + p[t - 1] + p[t + 1];
-        p[t] = 0.25 * (sum - h2 * rb[t]);
-      } else if (kk == kDir) {
-        p[t] = rb[t];
-      }
-    }
+// One node of a half-sweep: phi in shared memory at p, the rows' stride nx.
+__device__ __forceinline__ void relax_node(double* p, int nx, uint8_t kind, double f, double h2) {
+  const double s = p[-nx], n = p[nx], w = p[-1], e = p[1];
+  if (kind == kFluid) {
+    const double sum = s + n + w + e;
+    *p = 0.25 * fma(-h2, f, sum);      // written out: h2 * f must not be kept as a product
+  } else if (kind == kDir) {
+    *p = f;
+  }
 }
 
+// nu sweeps of one level in shared memory by one CTA of 32 warps: a warp takes a row, its lanes the row's
+// nodes of one colour.  A level of at most 66 x 66 nodes gives a thread two nodes of each colour at most;
+// their places, kinds and right-hand sides are then read once, and a half-sweep is the neighbours' loads,
+// the FP64 chain and a barrier.  (Narrower and longer levels take the loop over rows and lane groups.)
+__device__ __forceinline__ void cta_sweeps(double* p, const double* rb, const uint8_t* m, int nx, int ny, int nu,
+                                           double h2) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int NW = kCoarseThreads / 32;
+  if (nx <= 66 && ny <= 2 * NW + 2) {
+    int t[2][2];
+    double f[2][2];
+    uint8_t kind[2][2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int j = 1 + warp + NW * r, i = 1 + ((1 + j + c) & 1) + 2 * lane;
+        const bool in = j < ny - 1 && i < nx - 1;
+        t[r][c] = in ? j * nx + i : nx + 1;      // an interior node: its loads stay inside the level
+        f[r][c] = rb[t[r][c]];
+        kind[r][c] = in ? m[t[r][c]] : kFixed;
+      }
+    const bool two = 1 + warp + NW < ny - 1;
+#pragma unroll 1
+    for (int s = 0; s < nu; ++s)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        relax_node(p + t[0][c], nx, kind[0][c], f[0][c], h2);
+        if (two) relax_node(p + t[1][c], nx, kind[1][c], f[1][c], h2);
+        __syncthreads();
+      }
+    return;
+  }
+  for (int s = 0; s < 2 * nu; ++s) {
+    for (int j = 1 + warp; j < ny - 1; j += NW)
+      for (int i = 1 + ((1 + j + s) & 1) + 2 * lane; i < nx - 1; i += 64)
+        relax_node(p + j * nx + i, nx, m[j * nx + i], rb[j * nx + i], h2);
+    __syncthreads();
+  }
+}
+
+// The lower levels in one CTA.  Bound by the latency of the chain of half-sweeps and barriers on one SM
+// (65 x 65 and below with 2 + 2 sweeps, of which 385 x 257 uses 49 x 33: 20.5 -> 16.7 us, each sweep reading
+// its nodes' places, kinds and right-hand sides again before).
 __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   if (skip_launch(A.done)) return;
@@ -339,22 +391,22 @@ __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelA
   auto P = [&](int l) { return reinterpret_cast<double*>(smem + A.soff[l]); };
   auto RB = [&](int l) { return reinterpret_cast<double*>(smem + A.soff[l]) + A.nx[l] * A.ny[l]; };
   auto M = [&](int l) { return reinterpret_cast<uint8_t*>(smem + A.soff[l] + 16 * A.nx[l] * A.ny[l]); };
+  auto K = [&](int l) { return M(l) + A.nx[l] * A.ny[l]; };   // the reference's kinds (M: the smoother's)
   // stage the first level: phi, kinds, rhs (DIRICHLET: phi_bc)
   {
     const int nx = A.nx[0], ny = A.ny[0];
-    double* p = P(0); double* rb = RB(0); uint8_t* m = M(0);
+    double* p = P(0); double* rb = RB(0); uint8_t* m = M(0); uint8_t* kinds = K(0);
 #pragma unroll 4
     for (int j = warp; j < ny; j += nwarp)
       for (int i = lane; i < nx; i += 32) {
         const int k = j * nx + i;
         p[k] = A.phi[0][k];
         uint8_t kk = kFixed;
-        double v = 0.0;
-        if (i > 0 && j > 0 && i < nx - 1 && j < ny - 1) {
-          kk = smoother_kind(A.mask[0][k], A.bc[0] != nullptr);
-          v = kk == kFluid ? A.rhs[0][k] : kk == kDir ? A.bc[0][k] : 0.0;
-        }
-        m[k] = kk; rb[k] = v;
+        const uint8_t raw = A.mask[0][k];
+        double v = A.rhs[0][k];
+        if (i > 0 && j > 0 && i < nx - 1 && j < ny - 1) kk = smoother_kind(raw, A.bc[0] != nullptr);
+        if (kk != kFluid) v = kk == kDir ? A.bc[0][k] : 0.0;
+        m[k] = kk; rb[k] = v; kinds[k] = raw;
       }
   }
   __syncthreads();
@@ -362,20 +414,15 @@ __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelA
   int l = 0;
   for (;; ++l) {
     const int nx = A.nx[l], ny = A.ny[l];
-    for (int s = 0; s < 2 * A.nu1; ++s) {
-      cta_half_sweep(P(l), RB(l), M(l), nx, ny, s & 1, A.h2[l]);
-      __syncthreads();
-    }
+    cta_sweeps(P(l), RB(l), M(l), nx, ny, A.nu1, A.h2[l]);
     if (l == A.n - 1) break;
-    // restriction from the staged fine level; the kinds in shared memory are the smoother's,
-    // so the reference kinds come from global memory (level 0 of this CTA: the caller's;
-    // below it: what this CTA wrote, visible to the whole CTA after the barrier)
+    // restriction from the staged fine level
     const int nxc = A.nx[l + 1], nyc = A.ny[l + 1];
     const double* pf = P(l);
     const double* rbf = RB(l);
-    const uint8_t* mk = A.mask[l];   // reference kinds of level l (written above for l > 0)
-    const double h2i = 1.0 / A.h2[l];
-    double* pc = P(l + 1); double* rbc = RB(l + 1); uint8_t* mc = M(l + 1);
+    const uint8_t* mk = K(l);
+    const double h2i = A.h2i[l];
+    double* pc = P(l + 1); double* rbc = RB(l + 1); uint8_t* mc = M(l + 1); uint8_t* kinds_c = K(l + 1);
     for (int jc = warp; jc < nyc; jc += nwarp)
       for (int ic = lane; ic < nxc; ic += 32) {
         const int k = jc * nxc + ic;
@@ -401,6 +448,7 @@ __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelA
         A.rhs[l + 1][k] = fc;
         const uint8_t sk = interior ? smoother_kind(kc, A.bc[l + 1] != nullptr) : kFixed;
         mc[k] = sk;
+        kinds_c[k] = kc;
         rbc[k] = sk == kFluid ? fc : sk == kDir ? A.bc[l + 1][k] : 0.0;
       }
     __syncthreads();
@@ -417,10 +465,7 @@ __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelA
         if (m[k] == kFluid) p[k] += prolong_at(pc, nxc, i, j, A.bilinear != 0);
       }
     __syncthreads();
-    for (int s = 0; s < 2 * A.nu2; ++s) {
-      cta_half_sweep(p, RB(l), m, nx, ny, s & 1, A.h2[l]);
-      __syncthreads();
-    }
+    cta_sweeps(p, RB(l), m, nx, ny, A.nu2, A.h2[l]);
   }
   // every level's phi back to global memory (the reference keeps them in its level arrays)
   for (l = 0; l < A.n; ++l) {
@@ -431,39 +476,19 @@ __global__ void __launch_bounds__(kCoarseThreads) emb_coarse_kernel(CoarseLevelA
 }
 
 // ---------------------------------------------------------------- norms
-__device__ double cta_sum(double v, double* red) {
-  for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+// Sums of a and b over a CTA of 8 warps, in a fixed order, in thread 0.
+__device__ __forceinline__ void cta_sums(double& a, double& b, double (*red)[2]) {
+  for (int o = 16; o; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __syncthreads();
-  if (lane == 0) red[w] = v;
+  if (lane == 0) { red[w][0] = a; red[w][1] = b; }
   __syncthreads();
-  double s = 0.0;
+  a = b = 0.0;
   if (threadIdx.x == 0)
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += red[k];
-  return s;
-}
-
-// CTA b sums the interior rows 1 + b, 1 + b + gridDim.x, ... (threads along the row), so every
-// partial is formed in a fixed order.
-__global__ void __launch_bounds__(256) emb_norm_kernel(const double* __restrict__ phi, const double* __restrict__ rhs,
-                                                       const uint8_t* __restrict__ mask, int nx, int ny, double h2i,
-                                                       double* __restrict__ partials, const int* done) {
-  __shared__ double red[8];
-  if (skip_launch(done)) return;
-  double r2 = 0.0, f2 = 0.0;
-  for (int j = 1 + blockIdx.x; j < ny - 1; j += gridDim.x) {
-    const size_t row = (size_t)j * nx;
-    for (int i = 1 + threadIdx.x; i < nx - 1; i += 256) {
-      const size_t k = row + i;
-      if (mask[k] != kFluid) continue;
-      const double r = fine_residual(phi, rhs, mask, k, nx, h2i);
-      r2 += r * r;
-      f2 += rhs[k] * rhs[k];
-    }
-  }
-  const double a = cta_sum(r2, red);
-  const double b = cta_sum(f2, red);
-  if (threadIdx.x == 0) { partials[2 * blockIdx.x] = a; partials[2 * blockIdx.x + 1] = b; }
+    for (int k = 0; k < 8; ++k) { a += red[k][0]; b += red[k][1]; }
 }
 
 // What a solve knows of itself, on the device and (copied) on the host.
@@ -472,6 +497,7 @@ struct SolveState {
   double r0;           // ||r||^2 of the initial guess
   double rel, before;  // relative residual of the last check, and of the one before
   int cycles, done;
+  int ticket;          // CTAs of emb_norm_kernel that have left their partials
 };
 
 __device__ __forceinline__ double emb_relative(double r2, double f2, double r0) {
@@ -480,20 +506,48 @@ __device__ __forceinline__ double emb_relative(double r2, double f2, double r0) 
   return sqrt(r2);
 }
 
-// The norms from the partials in a fixed order.  cycle >= 0: they belong to a V-cycle of the solve, which
-// is counted and ends the solve below tol; -1: to the initial guess.
-__global__ void __launch_bounds__(256) emb_norm_final_kernel(const double* __restrict__ partials, int n,
-                                                             SolveState* __restrict__ S, int cycle, double tol,
-                                                             const int* done) {
-  __shared__ double red[8];
+// CTA b sums the interior rows 1 + b, 1 + b + gridDim.x, ... (threads along the row), so every
+// partial is formed in a fixed order; the CTA that finishes last adds the partials, in a fixed order too
+// (a launch of its own for that: 3 us).  cycle >= 0: the norms belong to a V-cycle of the solve, which is
+// counted and ends the solve below tol; -1: to the initial guess.
+__global__ void __launch_bounds__(256) emb_norm_kernel(const double* __restrict__ phi, const double* __restrict__ rhs,
+                                                       const uint8_t* __restrict__ mask, int nx, int ny, double h2i,
+                                                       double* partials, SolveState* S, int cycle, double tol,
+                                                       const int* done) {
+  __shared__ double red[8][2];
+  __shared__ bool last;
   if (skip_launch(done)) return;
   double a = 0.0, b = 0.0;
-  for (int k = threadIdx.x; k < n; k += 256) { a += partials[2 * k]; b += partials[2 * k + 1]; }
-  a = cta_sum(a, red);
-  b = cta_sum(b, red);
+  for (int j = 1 + blockIdx.x; j < ny - 1; j += gridDim.x) {
+    const size_t row = (size_t)j * nx;
+    for (int i = 1 + threadIdx.x; i < nx - 1; i += 256) {
+      const size_t k = row + i;
+      if (mask[k] != kFluid) continue;
+      const double r = fine_residual(phi, rhs, mask, k, nx, h2i);
+      a += r * r;
+      b += rhs[k] * rhs[k];
+    }
+  }
+  cta_sums(a, b, red);
   if (threadIdx.x == 0) {
+    partials[2 * blockIdx.x] = a;
+    partials[2 * blockIdx.x + 1] = b;
+    __threadfence();
+    last = atomicAdd(&S->ticket, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  a = b = 0.0;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += 256) {
+    a += __ldcg(partials + 2 * k);
+    b += __ldcg(partials + 2 * k + 1);
+  }
+  cta_sums(a, b, red);
+  if (threadIdx.x == 0) {
+    S->ticket = 0;
     S->r2 = a; S->f2 = b;
-    if (cycle < 0) { S->r0 = a; S->cycles = 0; S->done = 0; }
+    if (cycle < 0) S->r0 = a;
     S->before = S->rel;
     S->rel = emb_relative(a, b, S->r0);
     if (cycle >= 0) {
@@ -527,7 +581,7 @@ int coarse_smem_bytes(const EmbLevels& P, int l0, int offs[PIC_MAX_LEVELS]) {
   for (int l = l0; l < P.L; ++l) {
     offs[l - l0] = off;
     const int N = P.nx[l] * P.ny[l];
-    off += 16 * N + ((N + 15) / 16) * 16;
+    off += 16 * N + ((2 * N + 15) / 16) * 16;
   }
   return off;
 }
@@ -553,9 +607,9 @@ void launch_emb(void (*k)(KArgs...), dim3 grid, int block, size_t smem, cudaStre
 // restriction); rows = 0 where the tile kernels take it.  An item is one warp with FP64 chains to hide, so
 // a level needs about 14 of them per SM; the largest row count that still gives as many wastes
 // least on the rows a strip recomputes, up to 36 (more leave the last wave empty).  Measured on
-// B200, V-cycle at 4097^2 with at most 36 / 48 / 60 rows: 532 / 539 / 536 us at 14 items per SM, 532 /
-// 554 / 562 at 10, 589 / 591 / 592 at 18; tiles alone 772.  At 2049^2 238 against 273 us; at 1025^2 the
-// strips (10 per SM) would lose, 138 against 136.
+// B200, V-cycle with the line at 10 / 14 / 20 / 28 items per SM, and with tiles alone: 4097^2 494 / 488 /
+// 496 / 496, 755 us; 2049^2 202 / 200 / 203 / 206, 231; 1409^2 133 / 123 / 135 / 132, 132; 1025^2 (strips
+// only at 10) 100 / 95.  At most 36 rows: with 48 or 60 the 4097^2 V-cycle was 1 % slower.
 embs::Args strip_args(const EmbLevels& P, int l, int nu, bool down, const double* in, double* out) {
   constexpr int kItemsPerSm = 14, kMaxRows = 36;
   embs::Args A{};
@@ -700,6 +754,7 @@ int emb_vcycle(const EmbLevels& P, int l0, int nu1, int nu2, int options, cudaSt
       A.nx[k] = P.nx[l]; A.ny[k] = P.ny[l];
       A.phi[k] = P.phi[l]; A.rhs[k] = P.rhs[l]; A.mask[k] = P.mask[l]; A.bc[k] = P.bc[l];
       A.h2[k] = P.h * P.h * std::ldexp(1.0, 2 * l);
+      A.h2i[k] = 1.0 / A.h2[k];
     }
     const int bytes = coarse_smem_bytes(P, lc, A.soff);
     A.nu1 = nu1; A.nu2 = nu2; A.coarsen_any = any; A.bilinear = bilinear ? 1 : 0;
@@ -720,13 +775,12 @@ int emb_vcycle(const EmbLevels& P, int l0, int nu1, int nu2, int options, cudaSt
 
 namespace {
 
-// ||r||^2 and ||rhs||^2 over level 0's FLUID nodes into S; see emb_norm_final_kernel.
+// ||r||^2 and ||rhs||^2 over level 0's FLUID nodes into S; see emb_norm_kernel.
 int emb_norms(const EmbLevels& P, double* partials, SolveState* S, int cycle, double tol, cudaStream_t s) {
   const double h2i = 1.0 / (P.h * P.h);
   const int nb = std::max(1, std::min(kNormBlocks, P.ny[0] - 2));
   launch_emb(emb_norm_kernel, dim3(nb), 256, 0, s, (const double*)P.phi[0], (const double*)P.rhs[0],
-             (const uint8_t*)P.mask[0], P.nx[0], P.ny[0], h2i, partials, P.done);
-  launch_emb(emb_norm_final_kernel, dim3(1), 256, 0, s, (const double*)partials, nb, S, cycle, tol, P.done);
+             (const uint8_t*)P.mask[0], P.nx[0], P.ny[0], h2i, partials, S, cycle, tol, P.done);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return pic_fail(PIC_ERR_CUDA, cudaGetErrorString(e));
   return PIC_OK;
@@ -831,6 +885,8 @@ extern "C" int pic_solve_embedded_f64(double* phi, const double* rhs, const uint
   int cyc = 0;
   double rel = 0.0;
   if (check || relres_out) {
+    e = cudaMemsetAsync(S->state, 0, sizeof(SolveState), s);
+    if (e != cudaSuccess) return pic_fail(PIC_ERR_CUDA, cudaGetErrorString(e));
     if ((rc = emb_norms(P, S->partials, S->state, -1, tol, s))) return rc;
   }
   if (check) {
