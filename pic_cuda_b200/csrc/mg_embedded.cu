@@ -115,15 +115,15 @@ struct Tile {
 
 // NU sweeps of smooth_redblack on the interior tile nodes, colour (i + j) even first.  Thread k has one
 // node of each colour, the (k % H)-th one of its colour in row 1 + k / H (H = (W - 2) / 2 per row), and a
-// second pair 1024 nodes further on where the tile is that large (four sweeps): their kinds and right-hand sides stay in registers, and a half-sweep is four
-// shared loads, the FP64 chain and a barrier.  FLUID nodes relax, DIRICHLET nodes take their phi_bc when
-// the caller gave one, others stay.
+// second pair 1024 nodes further on where the tile is that large (four sweeps): their kinds and
+// right-hand sides stay in registers, and a half-sweep is four shared loads, the FP64 chain and a
+// barrier.  FLUID nodes relax, DIRICHLET nodes take their phi_bc when the caller gave one, others stay.
 template <int W, int NU>
 __device__ __forceinline__ void tile_sweeps(Tile<W>& T, double h2, bool has_bc) {
   if (NU == 0) return;
   constexpr int HW = W / 2, HALF = (W - 2) / 2, CNT = (W - 2) * HALF;
   constexpr int IT = (CNT + kSmoothThreads - 1) / kSmoothThreads;
-  int at[IT], par[IT];
+  int at[IT], par[IT];        // place of the pair in its row; tx parity of the colour-0 node
   double rb[IT][2];
   uint8_t m[IT][2];
 #pragma unroll
@@ -132,7 +132,7 @@ __device__ __forceinline__ void tile_sweeps(Tile<W>& T, double h2, bool has_bc) 
     const int r = k / HALF, ty = 1 + r;
     const int base = ty * HW + (k - r * HALF);
     at[it] = base;
-    par[it] = ty & 1;        // tx parity of colour 0 in row ty
+    par[it] = ty & 1;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int i = base + ((par[it] ^ c) ? 0 : 1);

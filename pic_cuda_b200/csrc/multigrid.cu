@@ -950,14 +950,16 @@ __global__ void __launch_bounds__(NT) mg_down_fast_kernel(const TileRef* __restr
 
 // Up leg (as mg_up_kernel modes 0 and 1).  MODE 0, level l >= 1: the bilinear prolongation
 // of the coarser correction added to the pre-smoothed one, NU post-sweeps, the owned nodes
-// to eu_l.  MODE 1, level 0 (NT = 256): the same with a one-node halo, then phi <- phi + e in
+// to eu_l.  MODE 1, level 0: the same with a one-node halo, then phi <- phi + e in
 // FP64, the new FP64 defect and the deterministic norm.  The e, f and coarse tiles arrive by
 // tensor-map loads; on level 0 phi64 (with a one-node halo) and rho of the owned nodes come
-// in one batch of asynchronous copies beside them.
+// in one batch of asynchronous copies beside them.  MODE 1 on 1024 threads, two CTAs per SM, where level 0
+// has at most wide_factor tiles per SM: its chain of copies, sweeps and the FP64 update is then shorter
+// (V-cycle at 257^2 28.7 -> 27.4 us, 513^2 40.4 -> 37.5; 129^2 22.8 -> 22.6).
 template <int NU, int MODE, int NT>
-__global__ void __launch_bounds__(NT, MODE ? 5 : 1) mg_up_fast_kernel(const TileRef* __restrict__ tiles,
-                                                                      const JobDev* __restrict__ jobs,
-                                                                      JobState* __restrict__ st, int l) {
+__global__ void __launch_bounds__(NT, MODE == 0 ? 1 : NT == 256 ? 5 : 2)
+    mg_up_fast_kernel(const TileRef* __restrict__ tiles, const JobDev* __restrict__ jobs, JobState* __restrict__ st,
+                      int l) {
   constexpr int H = 2 * NU, X = MODE, W = mgt::up_w(NU, X), OFF = mgt::up_off(NU, X), P = mgt::up_bw(NU, X);
   constexpr int CW = mgt::up_cw(NU, X), COFF = mgt::up_coff(NU, X), CP = mgt::up_cbw(NU, X);
   static_assert(W == kTU + 2 * H + 2 * X, "tile shape");
@@ -1086,7 +1088,7 @@ __global__ void __launch_bounds__(NT, MODE ? 5 : 1) mg_up_fast_kernel(const Tile
       }
     }
     __syncthreads();
-    double ar = 0.0;
+    double ar = 0.0, r_own = 0.0;
 #pragma unroll
     for (int u = 0; u < NO; ++u) {
       const int k = t + u * NT;
@@ -1104,7 +1106,20 @@ __global__ void __launch_bounds__(NT, MODE ? 5 : 1) mg_up_fast_kernel(const Tile
       }
       pn[g] = P64[q];
       f0[gy * pf + gx] = (float)r;
-      ar += r * r;
+      if constexpr (NT == 256) ar += r * r;
+      else r_own = r;
+    }
+    if constexpr (NT != 256) {   // the order of additions of 256 threads with four nodes each
+      static_assert(NO == 1, "one owned node per thread");
+      __syncthreads();           // rho in RH has been read
+      RH[t] = r_own;
+      __syncthreads();
+      if (t < 256)
+#pragma unroll
+        for (int u = 0; u < kTU * kTU / 256; ++u) {
+          const double r = RH[t + 256 * u];
+          ar += r * r;
+        }
     }
     // the tile's partial only: the job's norm, convergence test and buffer swap follow in
     // mg_finish_kernel, so no CTA waits for its stores or a shared ticket before it leaves
@@ -1186,7 +1201,8 @@ void launch_down_fast(int grid, bool wide, bool pdl, const TileRef* tiles, const
 template <int NU>
 void launch_up_fast(int grid, bool wide, bool pdl, const TileRef* tiles, const JobDev* jobs, JobState* st, int l,
                     int mode, cudaStream_t s) {
-  if (mode == 1) launch_k(mg_up_fast_kernel<NU, 1, 256>, grid, 256, 0, pdl, s, tiles, jobs, st, l);
+  if (mode == 1 && wide) launch_k(mg_up_fast_kernel<NU, 1, 1024>, grid, 1024, 0, pdl, s, tiles, jobs, st, l);
+  else if (mode == 1) launch_k(mg_up_fast_kernel<NU, 1, 256>, grid, 256, 0, pdl, s, tiles, jobs, st, l);
   else if (wide) launch_k(mg_up_fast_kernel<NU, 0, 1024>, grid, 1024, 0, pdl, s, tiles, jobs, st, l);
   else launch_k(mg_up_fast_kernel<NU, 0, 256>, grid, 256, 0, pdl, s, tiles, jobs, st, l);
 }
