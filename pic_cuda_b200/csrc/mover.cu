@@ -210,7 +210,7 @@ __global__ void chunk_table_kernel(const int* __restrict__ counts, const uint8_t
 
 // What a full step does before its particle pass, in one launch: the node field of every job, its charge
 // grid zeroed, the step's diagnostics reset and the work items counted.  (Four launches of 2-4 us each
-// before, most of it launch latency on small jobs: 129^2 step 123 -> 108 us together with the merged
+// before, most of it launch latency on small jobs: 129^2 step 123 -> 113 us together with the merged
 // V-cycle end and the memsets that moved into the solver's kernels.)
 __global__ void __launch_bounds__(256) step_head_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st,
                                                         const int* __restrict__ counts,
