@@ -955,7 +955,8 @@ __global__ void __launch_bounds__(NT) mg_down_fast_kernel(const TileRef* __restr
 // tensor-map loads; on level 0 phi64 (with a one-node halo) and rho of the owned nodes come
 // in one batch of asynchronous copies beside them.  MODE 1 on 1024 threads, two CTAs per SM, where level 0
 // has at most wide_factor tiles per SM: its chain of copies, sweeps and the FP64 update is then shorter
-// (V-cycle at 257^2 28.7 -> 27.4 us, 513^2 40.4 -> 37.5; 129^2 22.8 -> 22.6).
+// (V-cycle at 257^2 28.7 -> 27.4 us, 513^2 40.4 -> 37.5; 129^2 22.8 -> 22.6; at 1025^2, seven tiles per
+// SM, 256 threads stay the better ones, 56.8 against 66.4).
 template <int NU, int MODE, int NT>
 __global__ void __launch_bounds__(NT, MODE == 0 ? 1 : NT == 256 ? 5 : 2)
     mg_up_fast_kernel(const TileRef* __restrict__ tiles, const JobDev* __restrict__ jobs, JobState* __restrict__ st,
