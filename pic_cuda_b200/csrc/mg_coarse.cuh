@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kThreads) mg_coarse_reg_kernel(const int* __re
   tma::pdl_trigger();
   const int job = job_list[blockIdx.x];
   const JobDev& J = jobs[job];
-  if (st[job].converged) return;
+  if (st[job].converged) { tma::pdl_wait(); return; }   // waits all the same: see pdl_wait
   const int t = threadIdx.x, lc = J.lc, n = J.nl[lc], pitch = J.pl[lc];
   Params A;
   A.omega = J.omega;

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(32 * kWarps) mg_down_strip_kernel(const TileRe
   const TileRef tr = items[item];
   const JobDev& J = jobs[tr.job];
   const JobState& S = st[tr.job];
-  if (S.converged) return;
+  if (S.converged) { tma::pdl_wait(); return; }   // waits all the same: see pdl_wait
   DownArgs A;
   A.n = J.nl[l]; A.nc = J.nl[l + 1]; A.pf = J.pl[l]; A.pc = J.pl[l + 1];
   const double hl = J.h * (double)(1 << l);
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(32 * kWarps, MODE ? 4 : 5) mg_up_strip_kernel(
   const TileRef tr = items[item];
   const JobDev& J = jobs[tr.job];
   const JobState& S = st[tr.job];
-  if (S.converged) return;
+  if (S.converged) { tma::pdl_wait(); return; }   // waits all the same: see pdl_wait
   UpArgs A;
   A.n = J.nl[l]; A.nc = J.nl[l + 1]; A.pf = J.pl[l]; A.pc = J.pl[l + 1];
   const double hl = J.h * (double)(1 << l);

@@ -546,7 +546,7 @@ __device__ __forceinline__ void coarse_store(float* __restrict__ dst, const floa
 __device__ void coarse_solve(const int job, const JobDev* __restrict__ jobs, const JobState* __restrict__ st,
                              float* sm) {
   const JobDev& J = jobs[job];
-  if (st[job].converged) return;
+  if (st[job].converged) { tma::pdl_wait(); return; }   // waits all the same: see pdl_wait
   // The job's parameters are read once, before the first barrier: a barrier also orders the
   // compiler's view of global memory, so fields read through J afterwards would be reloaded.
   const int lc = J.lc, L = J.levels;
@@ -892,7 +892,7 @@ __global__ void __launch_bounds__(NT) mg_down_fast_kernel(const TileRef* __restr
   const TileRef tr = tiles[blockIdx.x];
   const JobDev& J = jobs[tr.job];
   const JobState& T = st[tr.job];
-  if (T.converged) return;
+  if (T.converged) { tma::pdl_wait(); return; }   // waits all the same: see pdl_wait
   const int nf = J.nl[l], nc = J.nl[l + 1], pf = J.pl[l], pc = J.pl[l + 1];
   const double hl = J.h * (double)(1 << l);
   const float h2 = (float)(hl * hl), inv_h2 = (float)(1.0 / (hl * hl));
@@ -985,7 +985,7 @@ __global__ void __launch_bounds__(NT, MODE == 0 ? 1 : NT == 256 ? 5 : 2)
   const TileRef tr = tiles[blockIdx.x];
   const JobDev& J = jobs[tr.job];
   JobState& T = st[tr.job];
-  if (T.converged) return;
+  if (T.converged) { tma::pdl_wait(); return; }   // waits all the same: see pdl_wait
   const int nf = J.nl[l], pf = J.pl[l];
   const double hl = J.h * (double)(1 << l);
   const float h2 = (float)(hl * hl);

@@ -82,6 +82,9 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // start while its predecessor in the stream is still running: it must call pdl_wait() before
 // reading anything the predecessor writes.  pdl_trigger() lets the successor launch once every
 // CTA of this kernel has called it (or exited).  Both are no-ops for ordinary launches.
+// pdl_wait() covers the launch directly before and no earlier one.  In a chain of such launches every CTA
+// must therefore wait, also one that leaves early with nothing to do: a launch whose CTAs all left
+// unwaited would end while its predecessor runs, and the launch behind it would start on unfinished data.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
