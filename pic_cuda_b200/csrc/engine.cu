@@ -43,6 +43,7 @@ namespace {
 
 constexpr int kMaxJobs = 4096;
 constexpr int kSlotsPerJob = 4;
+constexpr int kNumSms = 148;   // B200, where no device has been asked
 constexpr double kEps0 = 8.8541878128e-12;
 constexpr double kQe = 1.602176634e-19;
 constexpr double kKb = 1.380649e-23;
@@ -177,11 +178,39 @@ int event_capacity(const pic_job_config& c) {
   return (int)std::max<int64_t>(16384, std::min<int64_t>(ce / 128, 1 << 24));
 }
 
+// Rows per strip item of a level of the given sides (those of the jobs of a launch), 0 where the tile
+// kernels take the level.  An item is one warp, so a level needs about nine of them per SM to hide their
+// latency chains (twelve on the level-0 up kernel, whose tiles are better at 1025^2), and the largest row
+// count that still gives as many wastes least on the rows a strip recomputes before its first; beyond 72
+// rows the last wave costs more than that saves.  Measured on B200, V-cycle with strips against
+// tiles: 4097^2 277 / 401 us, 2049^2 121 / 139, 1025^2 62.6 / 63.3 (66.9 with the level-0 up as
+// strips too); forced at 513^2 67 / 46.5.  Rows per down item at 4097^2: 14 307 us, 30 301, 46 297,
+// 62 297, 94 300, 190 303; per level-0 up item: 12 338, 24 304, 48 289, 72 285, 96 294.
+int64_t strip_items(int n, int leg, int nu, int l, int rows) {
+  return (int64_t)(leg == 0 ? mg_down_strips(nu, n) : mg_up_strips(nu, l, n)) * ((n + rows - 1) / rows);
+}
+int strip_rows(int num_sms, const std::vector<int>& sides, int leg, int nu, int l) {
+  const int per_sm = leg == 1 && l == 0 ? 12 : 9;
+  for (int rows = mg_strip_rows(leg, nu, l, 72); rows > 0; rows = mg_strip_rows(leg, nu, l, rows - 1)) {
+    int64_t items = 0;
+    for (int n : sides) items += strip_items(n, leg, nu, l, rows);
+    if (items >= (int64_t)per_sm * num_sms) return rows;
+  }
+  return 0;
+}
+// Rows per strip item of a job's level-0 up leg.  This launch sums the job's residual norm, in an order that
+// follows the items, so the choice looks at the job alone: relres and the cycle a solve stops at must
+// not depend on the jobs beside it.  (Every other leg gives the same bits as tiles and as strips.)
+int up0_rows(int num_sms, int n, int nu) {
+  return nu >= 1 && nu <= kMaxFastNu ? strip_rows(num_sms, {n}, 1, nu, 0) : 0;
+}
+
 // FP64 partial sums of a job's level-0 launches: per init tile r^2, F^2 (pairs) and the charge, or a
-// pair per strip item of the level-0 up kernel (at most: the narrowest strips, the shortest rows).
-int64_t partials_bytes(int n) {
+// pair per strip item of the level-0 up kernel.
+int64_t partials_bytes(int num_sms, int n, int nu) {
   const int64_t t = (n + 31) / 32;
-  return std::max<int64_t>(24 * t * t, 16ll * mg_up_strips(kMaxFastNu, 0, n) * ((n + 7) / 8));
+  const int rows = up0_rows(num_sms, n, nu);
+  return std::max<int64_t>(24 * t * t, rows ? 16 * strip_items(n, 1, nu, 0, rows) : 0);
 }
 
 struct Layout {  // byte sizes of one job's device state
@@ -194,7 +223,8 @@ struct Layout {  // byte sizes of one job's device state
 // to coarse_top (<= PIC_COARSE_MAX) entirely in one CTA (lc = 0, the FP64 update then runs
 // as its own tile launch); otherwise the first level that fits one CTA, or a C-CTA cluster
 // when cluster_top asks for one above coarse_top.
-Layout job_layout(const pic_job_config& c, int cluster_C = 0, int cluster_top = 0, int coarse_top = PIC_COARSE_MAX) {
+Layout job_layout(const pic_job_config& c, int cluster_C = 0, int cluster_top = 0, int coarse_top = PIC_COARSE_MAX,
+                  int num_sms = kNumSms) {
   Layout L{};
   L.levels = c.mg_levels > 0 ? c.mg_levels : auto_levels(c.nx);
   const int one_cta = std::min(std::max(coarse_top, 3), PIC_COARSE_MAX);
@@ -220,7 +250,7 @@ Layout job_layout(const pic_job_config& c, int cluster_C = 0, int cluster_top = 
   for (int l = 1; l < L.levels; ++l) b += 4ll * mgt::round4(L.nl[l]) * L.nl[l];   // up-leg corrections
   b += 4ll * mgt::round4(c.nx) * c.ny;                                           // second level-0 rhs
   b += (int64_t)sizeof(CUtensorMap) * mgt::kTmapsPerLevel * L.levels;
-  b += partials_bytes(c.nx);
+  b += partials_bytes(num_sms, c.nx, c.nu_post);
   const int64_t ncells = (int64_t)(c.nx - 1) * (c.ny - 1) + 1;
   for (int s = 0; s < c.n_species; ++s) {
     const int64_t cap = round_up(std::max<int64_t>(c.species[s].capacity, 1), PIC_CHUNK);
@@ -244,7 +274,7 @@ struct pic_engine {
   // Job memory comes from a stream-ordered pool that keeps what jobs free for the next ones
   // (admitting and retiring jobs while others run should not cost a device-wide cudaFree).
   cudaMemPool_t pool = nullptr;
-  int num_sms = 148;
+  int num_sms = kNumSms;
   int mover_bps = 4;        // mover CTAs per SM: the occupancy limit
   int mover_cps = 0;        // PIC_OPT_MOVER_CTAS_PER_SM (0: mover_bps)
   int wide_factor = 2;      // PIC_OPT_MG_WIDE_TILES
@@ -428,28 +458,6 @@ void free_job(pic_engine* E, JobHost& J) {
   J.alive = false;
 }
 
-// Rows per strip item of level l for all jobs of a launch, 0 where the tile kernels take the level.
-// An item is one warp, so a level needs about nine of them per SM to hide their latency chains
-// (twelve on the level-0 up kernel, whose tiles are better at 1025^2), and the largest row count
-// that still gives as many wastes least on the rows a strip recomputes before its first; beyond 72
-// rows the last wave costs more than that saves.  Measured on B200, V-cycle with strips against
-// tiles: 4097^2 277 / 401 us, 2049^2 121 / 139, 1025^2 62.6 / 63.3 (66.9 with the level-0 up as
-// strips too); forced at 513^2 67 / 46.5.  Rows per down item at 4097^2: 14 307 us, 30 301, 46 297,
-// 62 297, 94 300, 190 303; per level-0 up item: 12 338, 24 304, 48 289, 72 285, 96 294.
-template <class F>
-int strip_rows(pic_engine* E, const std::vector<int>& ids, int l, F strips, int leg, int nu) {
-  const int per_sm = leg == 1 && l == 0 ? 12 : 9;
-  for (int rows = mg_strip_rows(leg, nu, l, 72); rows > 0; rows = mg_strip_rows(leg, nu, l, rows - 1)) {
-    int64_t items = 0;
-    for (int id : ids) {
-      const JobDev& D = E->jobs[id].dev;
-      if (l < D.lc) items += (int64_t)strips(D.nl[l]) * ((D.nl[l] + rows - 1) / rows);
-    }
-    if (items >= (int64_t)per_sm * E->num_sms) return rows;
-  }
-  return 0;
-}
-
 // Tile lists for the multigrid kernels over the given jobs.
 int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   out.release();
@@ -480,7 +488,7 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
       for (int tj = 0; tj < tc; ++tj)
         for (int ti = 0; ti < tc; ++ti) down[l].push_back({id, ti, tj, 0, 1, 0});
       const int tu = (D.nl[l] + 31) / 32;
-      for (int tj = 0; tj < tu; ++tj)
+      for (int tj = 0; l > 0 && tj < tu; ++tj)
         for (int ti = 0; ti < tu; ++ti) up[l].push_back({id, ti, tj, tj * tu + ti, tu * tu, 0});
     }
     if (E->cluster_C > 0 && D.nl[D.lc] > PIC_COARSE_MAX) {   // above one CTA's shared memory
@@ -494,30 +502,40 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   }
   const int fast_pre = (!ids.empty() && nu_pre_min == nu_pre_max && nu_pre_max <= kMaxFastNu) ? nu_pre_max : -1;
   const int fast_post = (!ids.empty() && nu_post_min == nu_post_max && nu_post_max <= kMaxFastNu) ? nu_post_max : -1;
-  std::vector<TileRef> sdown[PIC_MAX_LEVELS], sup[PIC_MAX_LEVELS];
-  int rows_down[PIC_MAX_LEVELS] = {}, rows_up[PIC_MAX_LEVELS] = {};
+  // strips of the level-0 up leg (by post-sweeps): job by job; the other jobs' tiles stay
+  std::vector<TileRef> sdown[PIC_MAX_LEVELS], sup[PIC_MAX_LEVELS], sup0[kMaxFastNu + 1];
+  auto add_items = [&](std::vector<TileRef>& v, int id, int leg, int nu, int l, int rows) {
+    const int n = E->jobs[id].dev.nl[l];
+    const int ts = leg == 0 ? mg_down_strips(nu, n) : mg_up_strips(nu, l, n), tr = (n + rows - 1) / rows;
+    for (int tj = 0; tj < tr; ++tj)
+      for (int ti = 0; ti < ts; ++ti) v.push_back({id, ti, tj, tj * ts + ti, rows, 0});
+    return tr * ts;
+  };
+  for (int id : ids) {
+    const JobDev& D = E->jobs[id].dev;
+    if (D.lc == 0) continue;
+    const int n = D.nl[0], rows = up0_rows(E->num_sms, n, D.nu_post), tu = (n + 31) / 32;
+    if (rows) {
+      finish.push_back(id);
+      finish.push_back(add_items(sup0[D.nu_post], id, 1, D.nu_post, 0, rows));
+      continue;
+    }
+    for (int tj = 0; tj < tu; ++tj)
+      for (int ti = 0; ti < tu; ++ti) up[0].push_back({id, ti, tj, tj * tu + ti, tu * tu, 0});
+    if (fast_post >= 0) { finish.push_back(id); finish.push_back(tu * tu); }
+  }
+  // strips of the other legs: where the level has enough items over all jobs
   for (int l = 0; l < max_depth; ++l)
     for (int leg = 0; leg < 2; ++leg) {
       const int nu = leg == 0 ? fast_pre : fast_post;
-      if (nu < 0) continue;
-      auto strips = [&](int n) { return leg == 0 ? mg_down_strips(nu, n) : mg_up_strips(nu, l, n); };
-      const int rows = strip_rows(E, ids, l, strips, leg, nu);
-      (leg == 0 ? rows_down : rows_up)[l] = rows;
-      for (int id : ids) {
-        const JobDev& D = E->jobs[id].dev;
-        if (l >= D.lc) continue;
-        const int n = D.nl[l];
-        if (rows == 0) {   // tile kernels
-          const int tu = (n + 31) / 32;
-          if (l == 0 && leg == 1) { finish.push_back(id); finish.push_back(tu * tu); }
-          continue;
-        }
-        const int ts = strips(n), tr = (n + rows - 1) / rows;
-        for (int tj = 0; tj < tr; ++tj)
-          for (int ti = 0; ti < ts; ++ti)
-            (leg == 0 ? sdown : sup)[l].push_back({id, ti, tj, tj * ts + ti, tr * ts, 0});
-        if (l == 0 && leg == 1) { finish.push_back(id); finish.push_back(tr * ts); }
-      }
+      if (nu < 0 || (leg == 1 && l == 0)) continue;
+      std::vector<int> sides;
+      for (int id : ids)
+        if (l < E->jobs[id].dev.lc) sides.push_back(E->jobs[id].dev.nl[l]);
+      const int rows = strip_rows(E->num_sms, sides, leg, nu, l);
+      if (!rows) continue;
+      for (int id : ids)
+        if (l < E->jobs[id].dev.lc) add_items((leg == 0 ? sdown : sup)[l], id, leg, nu, l, rows);
     }
   std::vector<TileRef> all;
   size_t off_init = all.size(); all.insert(all.end(), init.begin(), init.end());
@@ -528,6 +546,8 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   size_t off_sd[PIC_MAX_LEVELS], off_su[PIC_MAX_LEVELS];
   for (int l = 0; l < PIC_MAX_LEVELS; ++l) { off_sd[l] = all.size(); all.insert(all.end(), sdown[l].begin(), sdown[l].end()); }
   for (int l = 0; l < PIC_MAX_LEVELS; ++l) { off_su[l] = all.size(); all.insert(all.end(), sup[l].begin(), sup[l].end()); }
+  size_t off_s0[kMaxFastNu + 1];
+  for (int nu = 0; nu <= kMaxFastNu; ++nu) { off_s0[nu] = all.size(); all.insert(all.end(), sup0[nu].begin(), sup0[nu].end()); }
   if (!all.empty()) {
     CK(cudaMalloc(&out.d_tiles, all.size() * sizeof(TileRef)));
     CK(cudaMemcpy(out.d_tiles, all.data(), all.size() * sizeof(TileRef), cudaMemcpyHostToDevice));
@@ -547,9 +567,10 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   for (int l = 0; l < PIC_MAX_LEVELS; ++l) {
     M.down_tiles[l] = out.d_tiles + off_down[l]; M.n_down[l] = (int)down[l].size();
     M.up_tiles[l] = out.d_tiles + off_up[l]; M.n_up[l] = (int)up[l].size();
-    M.down_items[l] = out.d_tiles + off_sd[l]; M.n_down_items[l] = (int)sdown[l].size(); M.down_rows[l] = rows_down[l];
-    M.up_items[l] = out.d_tiles + off_su[l]; M.n_up_items[l] = (int)sup[l].size(); M.up_rows[l] = rows_up[l];
+    M.down_items[l] = out.d_tiles + off_sd[l]; M.n_down_items[l] = (int)sdown[l].size();
+    M.up_items[l] = out.d_tiles + off_su[l]; M.n_up_items[l] = (int)sup[l].size();
   }
+  for (int nu = 0; nu <= kMaxFastNu; ++nu) { M.up0_items[nu] = out.d_tiles + off_s0[nu]; M.n_up0_items[nu] = (int)sup0[nu].size(); }
   M.coarse_jobs = out.d_coarse; M.n_coarse = (int)coarse.size();
   M.cluster_jobs = out.d_coarse + coarse.size(); M.n_cluster = (int)cluster.size();
   M.finish_jobs = out.d_coarse + coarse.size() + cluster.size(); M.n_finish = (int)finish.size() / 2;
@@ -1068,7 +1089,7 @@ int pic_job_create(pic_engine* E, const pic_job_config* cfg, int* job_id) {
   for (int j = 0; j < kMaxJobs; ++j)
     if (!E->jobs[j].alive) { id = j; break; }
   if (id < 0) return fail(PIC_ERR_CAPACITY, "engine job table full");
-  const Layout lay = job_layout(*cfg, E->cluster_C, E->cluster_top, E->coarse_top);
+  const Layout lay = job_layout(*cfg, E->cluster_C, E->cluster_top, E->coarse_top, E->num_sms);
   if (E->pool_bytes > 0 && E->used_bytes + lay.total > E->pool_bytes) return fail(PIC_ERR_OOM, "engine memory budget exceeded");
   JobHost& J = E->jobs[id];
   J = JobHost();
@@ -1128,7 +1149,7 @@ int pic_job_create(pic_engine* E, const pic_job_config* cfg, int* job_id) {
     if (rc) { free_job(E, J); return rc; }
     D.tmaps = tm;
   }
-  ALLOC(D.partials, partials_bytes(c.nx));
+  ALLOC(D.partials, partials_bytes(E->num_sms, c.nx, c.nu_post));
   if (c.n_walls > 0) {
     std::vector<double> w(4 * c.n_walls);
     for (int k = 0; k < c.n_walls; ++k) {

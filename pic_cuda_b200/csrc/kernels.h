@@ -15,9 +15,9 @@
 // One multigrid tile of one job.
 struct TileRef {
   int job;
-  int ti, tj;     // tile origin in owned-node units (multiply by the tile size)
+  int ti, tj;     // tile origin in owned-node units (multiply by the tile size); strip items: strip, row chunk
   int local;      // index of this tile inside the job's tiles of the same launch
-  int nlocal;     // tiles of this job in the launch
+  int nlocal;     // tiles of this job in the launch; strip items: rows per item
   int pbase;      // first partial-sum slot of the job
 };
 
@@ -60,6 +60,8 @@ void launch_pid_max(const SlotDev* slot_dev, int64_t n, JobState* st, cudaStream
 int launch_sort_mask(const EngineLaunch& L, uint8_t* mask, int offset, cudaStream_t s);
 void launch_rho_sum(const JobDev* jd, JobState* st, double* scratch, int nparts, cudaStream_t s);
 
+// Largest smoothing count of the kernels with compile-time shapes.
+constexpr int kMaxFastNu = 4;
 // Multigrid (all jobs of a launch at once).
 struct MgLaunch {
   const TileRef* init_tiles; int n_init;                 // level-0 residual, 32x32 owned
@@ -69,10 +71,13 @@ struct MgLaunch {
   const TileRef* upd_tiles; int n_upd;                   // level-0 update for jobs with lc == 0
   const int* coarse_jobs; int n_coarse;                  // single-CTA coarse solve
   const int* cluster_jobs; int n_cluster;                // thread-block-cluster coarse solve
-  // strip items (mg_strips.cuh) and their rows per level, empty where the tile kernels take it
-  const TileRef* down_items[PIC_MAX_LEVELS]; int n_down_items[PIC_MAX_LEVELS]; int down_rows[PIC_MAX_LEVELS];
-  const TileRef* up_items[PIC_MAX_LEVELS]; int n_up_items[PIC_MAX_LEVELS]; int up_rows[PIC_MAX_LEVELS];
-  const int* finish_jobs; int n_finish;                  // (job, level-0 partials) of the jobs with lc >= 1
+  // strip items (mg_strips.cuh) per level, empty where the tile kernels take it
+  const TileRef* down_items[PIC_MAX_LEVELS]; int n_down_items[PIC_MAX_LEVELS];
+  const TileRef* up_items[PIC_MAX_LEVELS]; int n_up_items[PIC_MAX_LEVELS];   // levels >= 1
+  // level 0's up leg: strip items of the jobs large enough for them, by post-sweeps; up_tiles[0] holds
+  // the other jobs' tiles
+  const TileRef* up0_items[kMaxFastNu + 1]; int n_up0_items[kMaxFastNu + 1];
+  const int* finish_jobs; int n_finish;                  // (job, level-0 partials) where mg_finish_kernel ends the cycle
   int cluster_C;
   size_t cluster_smem;
   int max_depth;                                         // max lc over jobs
@@ -96,8 +101,6 @@ struct MgLevelsArgs {
   JobState* st;
   unsigned* gbar;
 };
-// Largest smoothing count of the kernels with compile-time shapes.
-constexpr int kMaxFastNu = 4;
 // Strip layout (mg_strips.cuh): strips across a level of side n, and the most rows per item, at most
 // `at_most`, that fill whole unrolled steps of the kernel (leg 0: down, 1: up; 0 if none does).
 int mg_down_strips(int nu, int n);

@@ -228,7 +228,7 @@ __device__ __forceinline__ void down_strip(const DownArgs& A, float2* ring) {
 template <int NU>
 __global__ void __launch_bounds__(32 * kWarps) mg_down_strip_kernel(const TileRef* __restrict__ items, int n_items,
                                                                     const JobDev* __restrict__ jobs,
-                                                                    const JobState* __restrict__ st, int l, int rows) {
+                                                                    const JobState* __restrict__ st, int l) {
   __shared__ __align__(16) float2 ring[kWarps][kDownRing * 32];
   constexpr int T = 2 * NU;
   tma::pdl_trigger();
@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(32 * kWarps) mg_down_strip_kernel(const TileRe
   if (item >= n_items) return;
   // item, job and job-state fields: none of them is written by the previous level's launch
   const TileRef tr = items[item];
+  const int rows = tr.nlocal;
   const JobDev& J = jobs[tr.job];
   const JobState& S = st[tr.job];
   if (S.converged) { tma::pdl_wait(); return; }   // waits all the same: see pdl_wait
@@ -455,7 +456,7 @@ __device__ __forceinline__ double up_strip(const UpArgs& A, UpStep<MODE>* ring) 
 template <int NU, int MODE>
 __global__ void __launch_bounds__(32 * kWarps, MODE ? 4 : 5) mg_up_strip_kernel(const TileRef* __restrict__ items, int n_items,
                                                                   const JobDev* __restrict__ jobs,
-                                                                  JobState* __restrict__ st, int l, int rows) {
+                                                                  JobState* __restrict__ st, int l) {
   __shared__ __align__(16) UpStep<MODE> ring[kWarps][up_ring(MODE)];
   constexpr int T = 2 * NU;
   tma::pdl_trigger();
@@ -464,6 +465,7 @@ __global__ void __launch_bounds__(32 * kWarps, MODE ? 4 : 5) mg_up_strip_kernel(
   // the job state changes only in mg_finish_kernel, at the end of a V-cycle (the next V-cycle's
   // first launch waits for it), so it is read before waiting for the previous launch
   const TileRef tr = items[item];
+  const int rows = tr.nlocal;
   const JobDev& J = jobs[tr.job];
   const JobState& S = st[tr.job];
   if (S.converged) { tma::pdl_wait(); return; }   // waits all the same: see pdl_wait

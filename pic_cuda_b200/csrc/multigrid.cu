@@ -1230,15 +1230,15 @@ void up_fast(int nu, int grid, bool wide, bool pdl, const TileRef* tiles, const 
 
 // Strip launches of one level for the sweep count every job of the launch shares.
 template <int NU>
-void down_strips(int n_items, const TileRef* items, bool pdl, const EngineLaunch& L, int l, int rows, cudaStream_t s) {
+void down_strips(int n_items, const TileRef* items, bool pdl, const EngineLaunch& L, int l, cudaStream_t s) {
   launch_k(mgs::mg_down_strip_kernel<NU>, (n_items + mgs::kWarps - 1) / mgs::kWarps, 32 * mgs::kWarps, 0, pdl, s, items,
-           n_items, L.jobs, (const JobState*)L.st, l, rows);
+           n_items, L.jobs, (const JobState*)L.st, l);
 }
 template <int NU>
-void up_strips(int n_items, const TileRef* items, bool pdl, const EngineLaunch& L, int l, int rows, cudaStream_t s) {
+void up_strips(int n_items, const TileRef* items, bool pdl, const EngineLaunch& L, int l, cudaStream_t s) {
   const int grid = (n_items + mgs::kWarps - 1) / mgs::kWarps;
-  if (l == 0) launch_k(mgs::mg_up_strip_kernel<NU, 1>, grid, 32 * mgs::kWarps, 0, pdl, s, items, n_items, L.jobs, L.st, l, rows);
-  else launch_k(mgs::mg_up_strip_kernel<NU, 0>, grid, 32 * mgs::kWarps, 0, pdl, s, items, n_items, L.jobs, L.st, l, rows);
+  if (l == 0) launch_k(mgs::mg_up_strip_kernel<NU, 1>, grid, 32 * mgs::kWarps, 0, pdl, s, items, n_items, L.jobs, L.st, l);
+  else launch_k(mgs::mg_up_strip_kernel<NU, 0>, grid, 32 * mgs::kWarps, 0, pdl, s, items, n_items, L.jobs, L.st, l);
 }
 
 // ---------------------------------------------------------------- levels 1 .. lc in one launch
@@ -1355,13 +1355,14 @@ int mg_strip_rows(int leg, int nu, int level, int at_most) { return mgs::rows_fi
 // Launch of one level.  When every job of the launch has the same smoothing count (<= kMaxFastNu):
 // the strip kernels where the level has enough items for them (strip_rows in engine.cu), else the
 // compile-time-shape tile kernels, on 1024-thread CTAs where a level has at most wide_factor
-// (default 2) tiles per SM.  Otherwise the generic tile kernels.  pdl: the launch follows a kernel
+// (default 2) tiles per SM.  Otherwise the generic tile kernels.  Level 0's up leg sums the residual norm
+// and chooses strips job by job (build_mg in engine.cu).  pdl: the launch follows a kernel
 // of the V-cycle that this one's prologue may overlap (programmatic serialisation).
 static bool launch_down(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, cudaStream_t s) {
   if (M.n_down_items[l]) {
     auto* f = M.fast_nu_pre == 0 ? down_strips<0> : M.fast_nu_pre == 1 ? down_strips<1> : M.fast_nu_pre == 2 ? down_strips<2>
               : M.fast_nu_pre == 3 ? down_strips<3> : down_strips<4>;
-    f(M.n_down_items[l], M.down_items[l], pdl && M.pdl, L, l, M.down_rows[l], s);
+    f(M.n_down_items[l], M.down_items[l], pdl && M.pdl, L, l, s);
     return true;
   }
   if (M.fast_nu_pre >= 0) {
@@ -1372,36 +1373,60 @@ static bool launch_down(const MgLaunch& M, int l, const EngineLaunch& L, bool pd
   mg_down_kernel<<<M.n_down[l], 256, down_smem(M.nu_pre_max), s>>>(M.down_tiles[l], L.jobs, L.st, l);
   return false;
 }
-static bool launch_up(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, const VcycleLoop* cond, cudaStream_t s) {
-  if (M.fast_nu_post < 0) {
-    mg_up_kernel<<<M.n_up[l], 256, up_smem(M.nu_post_max), s>>>(M.up_tiles[l], L.jobs, L.st, l, l == 0 ? 1 : 0,
-                                                                L.running);
-    return false;
-  }
+using StripLaunch = void (*)(int, const TileRef*, bool, const EngineLaunch&, int, cudaStream_t);
+static StripLaunch up_strips_of(int nu) {
+  return nu == 0 ? up_strips<0> : nu == 1 ? up_strips<1> : nu == 2 ? up_strips<2> : nu == 3 ? up_strips<3> : up_strips<4>;
+}
+static bool has_up(const MgLaunch& M, int l) {
+  bool any = M.n_up[l] || M.n_up_items[l];
+  if (l == 0)
+    for (int n : M.n_up0_items) any |= n != 0;
+  return any;
+}
+// Does mg_finish_kernel end the V-cycle of every job?
+static bool all_finish(const MgLaunch& M) {
+  return M.n_finish && !M.n_upd && !(M.n_up[0] && M.fast_nu_post < 0);
+}
+static bool launch_up(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, const VcycleLoop* cond, cudaStream_t s,
+                      int& k) {
+  if (l == 0)
+    for (int nu = 0; nu <= kMaxFastNu; ++nu)
+      if (M.n_up0_items[nu]) {
+        up_strips_of(nu)(M.n_up0_items[nu], M.up0_items[nu], pdl && M.pdl, L, 0, s);
+        pdl = true;
+        ++k;
+      }
   if (M.n_up_items[l]) {
-    auto* f = M.fast_nu_post == 0 ? up_strips<0> : M.fast_nu_post == 1 ? up_strips<1> : M.fast_nu_post == 2 ? up_strips<2>
-              : M.fast_nu_post == 3 ? up_strips<3> : up_strips<4>;
-    f(M.n_up_items[l], M.up_items[l], pdl && M.pdl, L, l, M.up_rows[l], s);
-  } else {
+    up_strips_of(M.fast_nu_post)(M.n_up_items[l], M.up_items[l], pdl && M.pdl, L, l, s);
+    pdl = true;
+    ++k;
+  } else if (M.n_up[l] && M.fast_nu_post >= 0) {
     up_fast(M.fast_nu_post, M.n_up[l], M.n_up[l] <= M.wide_factor * L.num_sms, pdl && M.pdl, M.up_tiles[l], L.jobs,
             L.st, l, l == 0 ? 1 : 0, s);
+    pdl = true;
+    ++k;
+  } else if (M.n_up[l]) {
+    mg_up_kernel<<<M.n_up[l], 256, up_smem(M.nu_post_max), s>>>(M.up_tiles[l], L.jobs, L.st, l, l == 0 ? 1 : 0,
+                                                                L.running);
+    pdl = false;
+    ++k;
   }
-  if (l == 0)
-    launch_k(mg_finish_kernel, M.n_finish, 1024, 0, M.pdl != 0, s, M.finish_jobs, L.jobs, L.st, L.running,
-             cond ? *cond : VcycleLoop{});
-  return true;
+  if (l == 0 && M.n_finish) {
+    launch_k(mg_finish_kernel, M.n_finish, 1024, 0, pdl && M.pdl, s, M.finish_jobs, L.jobs, L.st, L.running,
+             cond && all_finish(M) ? *cond : VcycleLoop{});
+    ++k;
+  }
+  return pdl;
 }
 
 int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, const VcycleLoop* cond, cudaStream_t s) {
   int k = 0;
   // the loop's condition in the last kernel where that is mg_finish_kernel, else after it
-  const bool fused = M.n_up[0] && M.fast_nu_post >= 0 && !M.n_upd;
   auto end_loop = [&]() {
-    if (!cond || fused) return;
+    if (!cond || all_finish(M)) return;
     vcycle_condition_kernel<<<1, 1, 0, s>>>(L.running, *cond);
     ++k;
   };
-  const VcycleLoop* const up_cond = fused ? cond : nullptr;
   if (M.levels_grid > 0 && M.max_depth >= 2 && !M.n_cluster) {
     if (M.n_down[0]) { launch_down(M, 0, L, false, s); ++k; }
     MgLevelsArgs a{};
@@ -1426,7 +1451,7 @@ int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, const VcycleLoop*
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, mg_levels_kernel, a);
     ++k;
-    if (M.n_up[0]) k += launch_up(M, 0, L, false, up_cond, s) ? 2 : 1;   // + mg_finish_kernel
+    if (has_up(M, 0)) launch_up(M, 0, L, false, cond, s, k);
     if (M.n_upd) { mg_up_kernel<<<M.n_upd, 256, up_smem(0), s>>>(M.upd_tiles, L.jobs, L.st, 0, 2, L.running); ++k; }
     end_loop();
     return k;
@@ -1448,7 +1473,7 @@ int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, const VcycleLoop*
   }
   if (M.n_cluster) { k += launch_mg_cluster(M.cluster_jobs, M.n_cluster, M.cluster_C, M.cluster_smem, L.jobs, L.st, s); prev_fast = false; }
   for (int l = M.max_depth - 1; l >= 0; --l)
-    if (M.n_up[l]) { prev_fast = launch_up(M, l, L, prev_fast, up_cond, s); k += (prev_fast && l == 0) ? 2 : 1; }
+    if (has_up(M, l)) prev_fast = launch_up(M, l, L, prev_fast, cond, s, k);
   if (M.n_upd) { mg_up_kernel<<<M.n_upd, 256, up_smem(0), s>>>(M.upd_tiles, L.jobs, L.st, 0, 2, L.running); ++k; }
   end_loop();
   return k;
