@@ -775,11 +775,12 @@ __global__ void __launch_bounds__(256) mg_up_kernel(const TileRef* __restrict__ 
     if (gx >= nf || gy >= nf) continue;
     const size_t g = (size_t)gy * nf + gx;
     const int q = (oy + 1) * PW + (ox + 1);
-    const double F = rhs_scale * rho[g];
+    const double rv = rho[g];
     double r = 0.0;
     if (gx > 0 && gx < nf - 1 && gy > 0 && gy < nf - 1) {
-      const double lap = (P[q - PW] + P[q + PW] + P[q - 1] + P[q + 1] - 4.0 * P[q]) * inv_h2;
-      r = F - lap;
+      const double lap = P[q - PW] + P[q + PW] + P[q - 1] + P[q + 1] - 4.0 * P[q];
+      // mode 1: as in the kernels with compile-time shapes, one of which a job gets when it is alone
+      r = mode == 1 ? mgs::defect(lap, inv_h2, rhs_scale, rv, gy) : rhs_scale * rv - lap * inv_h2;
     }
     pn[g] = P[q];
     f0[(size_t)gy * pf + gx] = (float)r;

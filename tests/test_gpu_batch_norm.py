@@ -46,3 +46,13 @@ def test_norm_does_not_depend_on_the_batch(jobs):
             assert b[1] == alone[1], (k, step)
             assert b[0] == alone[0], (k, step)
             np.testing.assert_array_equal(b[2], alone[2])
+
+
+# post-smoothing counts of which no kernel with compile-time shapes fits every job: the general kernel
+# runs jobs that have such a kernel when alone
+@pytest.mark.parametrize("jobs", [
+    [(257, 1e-7, 2, 2, 0), (257, 1e-7, 2, 3, 1), (129, 1e-7, 2, 2, 2), (129, 1e-7, 5, 6, 3)],
+    [(2049, 1e-5, 2, 2, 0), (257, 1e-7, 2, 3, 1), (65, 1e-8, 1, 1, 2)],
+], ids=["tiles", "tiles_and_strips"])
+def test_mixed_post_smoothing_keeps_each_result(jobs):
+    test_norm_does_not_depend_on_the_batch(jobs)
