@@ -238,8 +238,9 @@ int pic_job_diagnostics(pic_engine* e, int job, pic_diagnostics* out);
  *   default); applies to jobs created after the call.
  * PIC_OPT_MG_COARSE_TOP: largest level side (3..129) solved inside one CTA's shared memory
  *   (65 = default); applies to jobs created after the call.
- * PIC_OPT_MOVER_CTAS_PER_SM: CTAs per SM of the persistent particle pass (0 = as many as
- *   fit, the default; larger values are capped there).  Takes effect at the next step.
+ * PIC_OPT_MOVER_CTAS_PER_SM: warps per SM of the persistent particle pass, in CTAs of 256
+ *   threads (0 = as many as fit, the default; larger values are capped there: 28 warps, so 4
+ *   and more mean the same as 0).  Takes effect at the next step.
  * PIC_OPT_MG_WIDE_TILES: on multigrid tile levels with at most this many tiles per SM each
  *   tile runs on a 1024-thread CTA (a shorter latency chain when the level cannot fill the
  *   GPU), on the others on a 256-thread CTA (default 2; 0 = never).  Takes effect at the next

@@ -2,7 +2,7 @@
   * the multigrid launch shape (PIC_OPT_MG_LEVELS_KERNEL: one launch per level, or levels
     1..lc as one cooperative launch),
   * the counting-sort cadence of the jobs,
-  * the CTAs per SM of the persistent particle pass (PIC_OPT_MOVER_CTAS_PER_SM),
+  * the warps per SM of the persistent particle pass (PIC_OPT_MOVER_CTAS_PER_SM),
   * which multigrid levels run a tile per 1024-thread CTA (PIC_OPT_MG_WIDE_TILES).
 The knobs are tuned in turn (coordinate search): each knob's candidates are timed with the
 others at their best so far, and the fastest is kept.
@@ -22,7 +22,7 @@ from . import _lib as L
 class Tuner:
     levels_kernel: tuple = (0, 1)
     sort_every: tuple = (10, 20)
-    mover_ctas_per_sm: tuple = (0, 3)      # 0: as many as fit (4 at 64 registers)
+    mover_ctas_per_sm: tuple = (0, 3)      # 0: as many warps as fit (28); 3: 24
     mg_wide_tiles: tuple = (2, 0, 4)
     steps_per_trial: int = 6
     chosen: dict = field(default_factory=dict)

@@ -275,7 +275,7 @@ struct pic_engine {
   // (admitting and retiring jobs while others run should not cost a device-wide cudaFree).
   cudaMemPool_t pool = nullptr;
   int num_sms = kNumSms;
-  int mover_bps = 4;        // mover CTAs per SM: the occupancy limit
+  int mover_bps = 1;        // mover CTAs per SM: the occupancy limit (asked at creation)
   int mover_cps = 0;        // PIC_OPT_MOVER_CTAS_PER_SM (0: mover_bps)
   int wide_factor = 2;      // PIC_OPT_MG_WIDE_TILES
   int cluster_C = 0;          // thread-block cluster size of the coarse solver (0: none)
@@ -352,7 +352,7 @@ EngineLaunch make_launch(pic_engine* E, const uint8_t* active) {
   L.nslots = E->njobs_hw * kSlotsPerJob;
   L.njobs = E->njobs_hw;
   L.num_sms = E->num_sms;
-  L.mover_grid = E->num_sms * (E->mover_cps > 0 ? std::min(E->mover_cps, E->mover_bps) : E->mover_bps);
+  L.mover_grid = E->num_sms * mover_ctas(E->mover_cps, E->mover_bps);
   L.running = E->d_running;
   L.gbar = reinterpret_cast<unsigned*>(E->d_running + 2);  // the grid barrier's arrival counter
   L.absorbed = E->d_aux + 4 * kMaxJobs * kSlotsPerJob;

@@ -42,6 +42,13 @@ struct EngineLaunch {
 };
 
 int mover_blocks_per_sm();
+// Particle-pass CTAs (of PIC_MOVER_THREADS) per SM for a value of PIC_OPT_MOVER_CTAS_PER_SM, which counts
+// CTAs of 256 threads whatever the kernel's CTA size is; fit: as many as an SM holds (0 asks for them).
+constexpr int kMoverOptionThreads = 256;
+inline int mover_ctas(int option, int fit) {
+  const int ctas = option * (kMoverOptionThreads / PIC_MOVER_THREADS);
+  return option > 0 && ctas < fit ? ctas : fit;
+}
 // Before a full step's particle pass: the node field, zero charge, reset diagnostics, work items.
 int launch_step_head(const EngineLaunch& L, cudaStream_t s);
 // after_head: launch_step_head ran before it (the pass needs neither the node field nor the items).
