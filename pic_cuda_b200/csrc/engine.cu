@@ -72,7 +72,7 @@ struct JobHost {
   int64_t bytes = 0;
   int64_t steps = 0;
   bool pending = false;
-  bool loaded = false;     // particles were loaded since the job's last sort (in no cell order)
+  bool fresh[kSlotsPerJob] = {};   // particles were loaded since the slot's last sort (in no cell order)
   // JobState::total_charge holds the sum of the present rho: the level-0 residual kernel
   // of every field solve computes it; entry points that change rho otherwise clear this
   bool charge_fresh = false;
@@ -726,22 +726,29 @@ int check_job(pic_engine* E, int job) {
 }
 
 // One full step of every live job.
+// Marks a job's slots in a sort mask, the freshly loaded ones as such (their flag is cleared: the sort follows);
+// true if there are any of those.
+bool mark_sort(JobHost& J, uint8_t* mask) {
+  bool fresh = false;
+  for (int k = 0; k < J.cfg.n_species; ++k) {
+    mask[k] = J.fresh[k] ? kSortDue | kSortFresh : kSortDue;
+    fresh |= J.fresh[k];
+    J.fresh[k] = false;
+  }
+  return fresh;
+}
 // Counting sort (stream-ordered on s) of the jobs for which `due` holds.
 template <typename Due>
 int sort_jobs(pic_engine* E, const EngineLaunch& L, Due due, cudaStream_t s, bool* launched) {
   std::vector<uint8_t> mask(L.nslots, 0);
-  bool any = false, loaded = false;
+  bool any = false, fresh = false;
   int max_cells = 0;
   int64_t max_p = 0;
   for (int j = 0; j < E->njobs_hw; ++j) {
     JobHost& J = E->jobs[j];
     if (!J.alive || J.cfg.sort_every <= 0 || !due(J)) continue;
-    loaded |= J.loaded;
-    J.loaded = false;
-    for (int k = 0; k < J.cfg.n_species; ++k) {
-      mask[j * kSlotsPerJob + k] = 1;
-      max_p = std::max<int64_t>(max_p, J.cfg.species[k].capacity);
-    }
+    fresh |= mark_sort(J, mask.data() + j * kSlotsPerJob);
+    for (int k = 0; k < J.cfg.n_species; ++k) max_p = std::max<int64_t>(max_p, J.cfg.species[k].capacity);
     max_cells = std::max(max_cells, J.dev.ncx * J.dev.ncy);
     any = true;
   }
@@ -749,7 +756,7 @@ int sort_jobs(pic_engine* E, const EngineLaunch& L, Due due, cudaStream_t s, boo
   if (!any) return PIC_OK;
   CK(cudaMemcpyAsync(E->d_mask, mask.data(), mask.size(), cudaMemcpyHostToDevice, s));
   phase_mark(E, 0, true, s);
-  E->launches += launch_sort(L, E->d_mask, max_cells, (int)std::min<int64_t>(max_p, 1 << 30), true, loaded, s);
+  E->launches += launch_sort(L, E->d_mask, max_cells, (int)std::min<int64_t>(max_p, 1 << 30), true, fresh, s);
   phase_mark(E, 0, false, s);
   return PIC_OK;
 }
@@ -1388,7 +1395,7 @@ int pic_job_load_species(pic_engine* E, int job, int species, int64_t n, const d
   const SlotDev* sd = E->d_slots + job * kSlotsPerJob + species;
   launch_load_species(sd, nullptr, n, dx_, dy_, dvx, dvy, dvz, dpid, hs.next_pid, 1.0 / dxv, 1.0 / dyv, J.dev.ncx,
                       J.dev.ncy, s);
-  J.loaded = true;
+  J.fresh[species] = true;
   const int ni = (int)n;
   CK(cudaMemcpyAsync(E->d_counts + job * kSlotsPerJob + species, &ni, sizeof(int), cudaMemcpyHostToDevice, s));
   if (dpid) {
@@ -1529,13 +1536,25 @@ int pic_step_graph(pic_engine* E, int nsteps, void* stream) {
     bool sorted = false;
     rc = sort_jobs(E, make_launch(E, nullptr), sort_before_first, s, &sorted);
     if (rc) return rc;
-    bool sort_due = false;
+    // the sort due after the step is in the graph, except that of large slots loaded in the middle of a
+    // run: it is rare, takes the band pass and follows the graph
+    bool sort_due = false, fresh = false;
     for (int j = 0; j < E->njobs_hw; ++j) {
-      const JobHost& J = E->jobs[j];
-      if (J.alive && J.cfg.sort_every > 0 && sort_after(J)) sort_due = true;
+      JobHost& J = E->jobs[j];
+      if (!J.alive || J.cfg.sort_every <= 0 || !sort_after(J)) continue;
+      sort_due = true;
+      for (int q = 0; q < J.cfg.n_species; ++q) {
+        J.fresh[q] = J.fresh[q] && J.cfg.species[q].capacity >= kBandMinParticles;
+        fresh |= J.fresh[q];
+      }
     }
-    CK(cudaGraphLaunch(sort_due ? E->graph_exec_sort : E->graph_exec, s));
-    E->launches += E->graph_fixed_launches[sort_due ? 1 : 0];
+    const bool in_graph = sort_due && !fresh;
+    CK(cudaGraphLaunch(in_graph ? E->graph_exec_sort : E->graph_exec, s));
+    E->launches += E->graph_fixed_launches[in_graph ? 1 : 0];
+    if (fresh) {
+      rc = sort_jobs(E, make_launch(E, nullptr), sort_after, s, &sorted);
+      if (rc) return rc;
+    }
     E->graph_steps++;
     E->steps_taken++;
     for (int j = 0; j < E->njobs_hw; ++j)
@@ -1686,14 +1705,14 @@ int pic_job_sort(pic_engine* E, int job, void* stream) {
   if (rc) return rc;
   CK(cudaSetDevice(E->device));
   cudaStream_t s = pick(E, stream);
-  rc = job_mask(E, job, s);
-  if (rc) return rc;
   JobHost& J = E->jobs[job];
+  std::vector<uint8_t> mask(E->njobs_hw * kSlotsPerJob, 0);
+  const bool fresh = mark_sort(J, mask.data() + job * kSlotsPerJob);
+  CK(cudaMemcpyAsync(E->d_mask, mask.data(), mask.size(), cudaMemcpyHostToDevice, s));
   int64_t maxp = 0;
   for (int k = 0; k < J.cfg.n_species; ++k) maxp = std::max<int64_t>(maxp, J.cfg.species[k].capacity);
   EngineLaunch L = make_launch(E, nullptr);
-  launch_sort(L, E->d_mask, J.dev.ncx * J.dev.ncy, (int)std::min<int64_t>(maxp, 1 << 30), false, J.loaded, s);
-  J.loaded = false;
+  launch_sort(L, E->d_mask, J.dev.ncx * J.dev.ncy, (int)std::min<int64_t>(maxp, 1 << 30), false, fresh, s);
   CK(cudaStreamSynchronize(s));
   CK(cudaGetLastError());
   return PIC_OK;

@@ -16,9 +16,6 @@
 namespace {
 
 constexpr int kTile = 2048;     // cells per scan tile (256 threads x 8)
-// Freshly loaded slots of at least this many particles take the band pass (below, a slot's arrays sit
-// in L2 anyway: 1.3 M particles 0.224 ms without it, 0.229 with; 2.6 M 0.456 and 0.435).
-constexpr int kBandMinParticles = 2000000;
 
 __device__ __forceinline__ uint32_t dense_key(uint32_t c, int ncx, uint32_t ncells) {
   return c == PIC_CELL_OUT ? ncells : (uint32_t)cell_j(c) * (uint32_t)ncx + (uint32_t)cell_i(c);
@@ -294,8 +291,8 @@ constexpr int kBandChunk = kBandThreads * kBandPer;
 constexpr int kBandSums = (kBands + 1 + 31) / 32;         // bands per lane of the scan
 
 __device__ __forceinline__ int bands_of(const JobDev& J) { return min(kBands, J.ncy); }
-__device__ __forceinline__ bool banded_slot(const JobDev& J, int n) {
-  return n >= kBandMinParticles && J.ncx * J.ncy >= 4 * kBands;
+__device__ __forceinline__ bool banded_slot(uint8_t mask, const JobDev& J, int n) {
+  return (mask & kSortFresh) && n >= kBandMinParticles && J.ncx * J.ncy >= 4 * kBands;
 }
 // band of a cell: rows split into nb bands; particles outside the grid go last
 __device__ __forceinline__ int band_of(uint32_t c, int ncy, int nb) {
@@ -308,7 +305,7 @@ __global__ void sort_band_init(const JobDev* jobs, const SlotDev* slots, const i
   if (!mask[s]) return;
   const SlotDev& S = slots[s];
   const JobDev& J = jobs[S.job];
-  if (!banded_slot(J, counts[s])) return;
+  if (!banded_slot(mask[s], J, counts[s])) return;
   const int nb = bands_of(J);
   for (int b = threadIdx.x; b <= nb; b += blockDim.x) {
     const int row = b == nb ? J.ncy : (b * J.ncy + nb - 1) / nb;   // the band's first row
@@ -323,7 +320,7 @@ __global__ void __launch_bounds__(kBandThreads) sort_band_scatter(const JobDev* 
   const SlotDev& S = slots[s];
   const JobDev& J = jobs[S.job];
   const int n = counts[s];
-  if (!banded_slot(J, n)) return;
+  if (!banded_slot(mask[s], J, n)) return;
   __shared__ int h[kBands + 1], off[32 * kBandSums], base[kBands + 1];
   __shared__ int place[kBandChunk];
   __shared__ uint32_t stage[2][kBandChunk];
@@ -411,7 +408,7 @@ __global__ void sort_band_swap(const JobDev* jobs, SlotDev* slots, const int* co
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nslots || !mask[s]) return;
   SlotDev& S = slots[s];
-  if (!banded_slot(jobs[S.job], counts[s])) return;
+  if (!banded_slot(mask[s], jobs[S.job], counts[s])) return;
   swp(S.cell, S.cell_b); swp(S.fx, S.fx_b); swp(S.fy, S.fy_b);
   swp(S.vx, S.vx_b); swp(S.vy, S.vy_b); swp(S.vz, S.vz_b); swp(S.pid, S.pid_b);
 }
@@ -433,7 +430,7 @@ __global__ void sort_mask_kernel(const JobDev* jobs, const JobState* st, const u
   const int j = s / PIC_MAX_SPECIES;
   const JobDev& J = jobs[j];
   const bool due = active[s] && J.sort_every > 0 && ((st[j].step + offset) % J.sort_every) == 0;
-  mask[s] = due ? 1 : 0;
+  mask[s] = due ? kSortDue : 0;
 }
 
 }  // namespace
