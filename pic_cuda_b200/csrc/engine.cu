@@ -396,7 +396,7 @@ int encode_level_map(CUtensorMap* m, const float* base, int n, int pitch, int bw
 }
 
 // The tile tensor maps of every level the tile kernels process (levels above the coarse
-// solver's; mg_tiles.h lists them), copied to `dst` on the device.  Sweep counts above the
+// solver's; mg_tiles.h lists them), copied to `dst` on the device.  Sweep counts without
 // compile-time shapes run on the generic kernels, which read global memory directly.
 int make_tile_maps(const JobDev& D, int nu_pre, int nu_post, CUtensorMap* dst) {
   std::vector<CUtensorMap> maps((size_t)mgt::kTmapsPerLevel * D.levels);
@@ -405,12 +405,12 @@ int make_tile_maps(const JobDev& D, int nu_pre, int nu_post, CUtensorMap* dst) {
   for (int l = 0; l < D.lc && !rc; ++l) {
     CUtensorMap* m = maps.data() + (size_t)mgt::kTmapsPerLevel * l;
     const int n = D.nl[l], p = D.pl[l];
-    if (nu_pre <= 4) {
+    if (nu_pre >= 1 && nu_pre <= kMaxFastNu) {
       const int bw = mgt::down_bw(nu_pre), bh = mgt::down_w(nu_pre);
       rc = encode_level_map(m + mgt::kMapDownF, D.f[l], n, p, bw, bh);
       if (!rc && l == 0) rc = encode_level_map(m + mgt::kMapDownF0b, D.f0b, n, p, bw, bh);
     }
-    if (!rc && nu_post <= 4) {
+    if (!rc && nu_post >= 1 && nu_post <= kMaxFastNu) {
       const int x = l == 0 ? 1 : 0;
       const int bw = mgt::up_bw(nu_post, x), bh = mgt::up_w(nu_post, x);
       rc = encode_level_map(m + mgt::kMapUpE, D.e[l], n, p, bw, bh);
@@ -500,8 +500,9 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
       coarse_smem = std::max(coarse_smem, mg_coarse_smem(D.nl, D.lc, D.levels));
     }
   }
-  const int fast_pre = (!ids.empty() && nu_pre_min == nu_pre_max && nu_pre_max <= kMaxFastNu) ? nu_pre_max : -1;
-  const int fast_post = (!ids.empty() && nu_post_min == nu_post_max && nu_post_max <= kMaxFastNu) ? nu_post_max : -1;
+  // the count every job has, where kernels with compile-time shapes exist for it (the maxima start at 1)
+  const int fast_pre = nu_pre_min == nu_pre_max && nu_pre_max <= kMaxFastNu ? nu_pre_max : -1;
+  const int fast_post = nu_post_min == nu_post_max && nu_post_max <= kMaxFastNu ? nu_post_max : -1;
   // strips of the level-0 up leg (by post-sweeps): job by job; the other jobs' tiles stay
   std::vector<TileRef> sdown[PIC_MAX_LEVELS], sup[PIC_MAX_LEVELS], sup0[kMaxFastNu + 1];
   auto add_items = [&](std::vector<TileRef>& v, int id, int leg, int nu, int l, int rows) {

@@ -72,7 +72,8 @@ void launch_pid_max(const SlotDev* slot_dev, int64_t n, JobState* st, cudaStream
 int launch_sort_mask(const EngineLaunch& L, uint8_t* mask, int offset, cudaStream_t s);
 void launch_rho_sum(const JobDev* jd, JobState* st, double* scratch, int nparts, cudaStream_t s);
 
-// Largest smoothing count of the kernels with compile-time shapes.
+// Largest smoothing count of the kernels with compile-time shapes (from one sweep on; none runs on the
+// general ones).
 constexpr int kMaxFastNu = 4;
 // Multigrid (all jobs of a launch at once).
 struct MgLaunch {

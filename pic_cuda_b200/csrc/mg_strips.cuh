@@ -138,7 +138,8 @@ __device__ __forceinline__ void down_strip(const DownArgs& A, float2* ring) {
     ++next;
   };
   // the row the last half-sweep has just completed, and the coarse row, of a row step
-  constexpr int kDone = NU > 0 ? T - 1 : 0;
+  static_assert(NU > 0, "without sweeps the general kernels run");
+  constexpr int kDone = T - 1;
   float* eout = A.e + ((ptrdiff_t)(js - kDone) * pf + c0);
   float* cout = A.fc + ((ptrdiff_t)((js - T) >> 1) * A.pc + (c0 >> 1));
   float E[WIN + D][2], F[WIN + D][2];
@@ -192,12 +193,9 @@ __device__ __forceinline__ void down_strip(const DownArgs& A, float2* ring) {
       float rc[3];
       {
         const int b = a - T;
-        float l0 = 0.f, l1 = 0.f;
-        if (NU > 0) {
-          const float w = left_of(E[b][1]), e = right_of(E[b][0]);
-          l0 = E[b - 1][0] + E[b + (NU > 0)][0] + w + E[b][1] - 4.f * E[b][0];
-          l1 = E[b - 1][1] + E[b + (NU > 0)][1] + E[b][0] + e - 4.f * E[b][1];
-        }
+        const float w = left_of(E[b][1]), e = right_of(E[b][0]);
+        const float l0 = E[b - 1][0] + E[b + 1][0] + w + E[b][1] - 4.f * E[b][0];
+        const float l1 = E[b - 1][1] + E[b + 1][1] + E[b][0] + e - 4.f * E[b][1];
         rc[1] = fmaf(-l0, inv_h2, F[b][0]);
         rc[2] = fmaf(-l1, inv_h2, F[b][1]);
         rc[0] = left_of(rc[2]);

@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(256) mg_up_kernel(const TileRef* __restrict__ 
 }
 
 // ---------------------------------------------------------------- tile kernels, compile-time shapes
-// The per-level launches of the V-cycle for a uniform smoothing count NU (0..4): the tile
+// The per-level launches of the V-cycle for a uniform smoothing count NU (1..4): the tile
 // width W is a compile-time constant, so every global input of a tile is requested in one
 // unrolled batch of asynchronous copies (one memory latency per tile instead of one per row),
 // and the sweeps use the column-per-thread red-black mapping of the coarse solver on an even
@@ -1211,7 +1211,6 @@ void launch_up_fast(int grid, bool wide, bool pdl, const TileRef* tiles, const J
 void down_fast(int nu, int grid, bool wide, bool pdl, const TileRef* tiles, const JobDev* jobs, const JobState* st,
                int l, cudaStream_t s) {
   switch (nu) {
-    case 0: launch_down_fast<0>(grid, wide, pdl, tiles, jobs, st, l, s); break;
     case 1: launch_down_fast<1>(grid, wide, pdl, tiles, jobs, st, l, s); break;
     case 2: launch_down_fast<2>(grid, wide, pdl, tiles, jobs, st, l, s); break;
     case 3: launch_down_fast<3>(grid, wide, pdl, tiles, jobs, st, l, s); break;
@@ -1221,7 +1220,6 @@ void down_fast(int nu, int grid, bool wide, bool pdl, const TileRef* tiles, cons
 void up_fast(int nu, int grid, bool wide, bool pdl, const TileRef* tiles, const JobDev* jobs, JobState* st, int l,
              int mode, cudaStream_t s) {
   switch (nu) {
-    case 0: launch_up_fast<0>(grid, wide, pdl, tiles, jobs, st, l, mode, s); break;
     case 1: launch_up_fast<1>(grid, wide, pdl, tiles, jobs, st, l, mode, s); break;
     case 2: launch_up_fast<2>(grid, wide, pdl, tiles, jobs, st, l, mode, s); break;
     case 3: launch_up_fast<3>(grid, wide, pdl, tiles, jobs, st, l, mode, s); break;
@@ -1353,7 +1351,7 @@ int mg_up_strips(int nu, int level, int n) { return mgs::up_strips(nu, level == 
 int mg_strip_rows(int leg, int nu, int level, int at_most) { return mgs::rows_fit(leg, nu, level == 0 ? 1 : 0, at_most); }
 
 
-// Launch of one level.  When every job of the launch has the same smoothing count (<= kMaxFastNu):
+// Launch of one level.  When every job of the launch has the same smoothing count (1 .. kMaxFastNu):
 // the strip kernels where the level has enough items for them (strip_rows in engine.cu), else the
 // compile-time-shape tile kernels, on 1024-thread CTAs where a level has at most wide_factor
 // (default 2) tiles per SM.  Otherwise the generic tile kernels.  Level 0's up leg sums the residual norm
@@ -1361,8 +1359,8 @@ int mg_strip_rows(int leg, int nu, int level, int at_most) { return mgs::rows_fi
 // of the V-cycle that this one's prologue may overlap (programmatic serialisation).
 static bool launch_down(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, cudaStream_t s) {
   if (M.n_down_items[l]) {
-    auto* f = M.fast_nu_pre == 0 ? down_strips<0> : M.fast_nu_pre == 1 ? down_strips<1> : M.fast_nu_pre == 2 ? down_strips<2>
-              : M.fast_nu_pre == 3 ? down_strips<3> : down_strips<4>;
+    auto* f = M.fast_nu_pre == 1 ? down_strips<1> : M.fast_nu_pre == 2 ? down_strips<2> : M.fast_nu_pre == 3 ? down_strips<3>
+                                                                                                           : down_strips<4>;
     f(M.n_down_items[l], M.down_items[l], pdl && M.pdl, L, l, s);
     return true;
   }
@@ -1376,7 +1374,7 @@ static bool launch_down(const MgLaunch& M, int l, const EngineLaunch& L, bool pd
 }
 using StripLaunch = void (*)(int, const TileRef*, bool, const EngineLaunch&, int, cudaStream_t);
 static StripLaunch up_strips_of(int nu) {
-  return nu == 0 ? up_strips<0> : nu == 1 ? up_strips<1> : nu == 2 ? up_strips<2> : nu == 3 ? up_strips<3> : up_strips<4>;
+  return nu == 1 ? up_strips<1> : nu == 2 ? up_strips<2> : nu == 3 ? up_strips<3> : up_strips<4>;
 }
 static bool has_up(const MgLaunch& M, int l) {
   bool any = M.n_up[l] || M.n_up_items[l];
@@ -1391,7 +1389,7 @@ static bool all_finish(const MgLaunch& M) {
 static bool launch_up(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, const VcycleLoop* cond, cudaStream_t s,
                       int& k) {
   if (l == 0)
-    for (int nu = 0; nu <= kMaxFastNu; ++nu)
+    for (int nu = 1; nu <= kMaxFastNu; ++nu)
       if (M.n_up0_items[nu]) {
         up_strips_of(nu)(M.n_up0_items[nu], M.up0_items[nu], pdl && M.pdl, L, 0, s);
         pdl = true;
