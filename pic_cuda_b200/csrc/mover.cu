@@ -63,48 +63,30 @@ __device__ __forceinline__ void neutral_velocity(uint64_t seed, uint32_t pid, ui
 
 }  // namespace
 
-// Particles per lane and per warp work item: an item is kPPL / 2 blocks of 64 consecutive
-// particles, and lane l of a warp holds particles 2 l and 2 l + 1 of each block in registers, loaded
-// with one vector load per array and block (contiguous per warp).  The deposit sums block by block
-// (its FP32 rounding depends on the blocks, not on how many an item has).  Capacities are multiples
-// of PIC_CHUNK, so every item lies inside the arrays.  Small CTAs let the register file hold 28
-// warps of 72 registers.  Measured on B200, ms per pass at 1025^2 (2e7 particles, FP32 deposit) /
-// 4097^2 (2e8) / 4097^2 with the int64 deposit: one block, 128 threads x 7 CTAs per SM 0.341 / 3.22 /
-// 3.50; x 6 0.352 / 3.40 / 3.67; x 8 0.361 / 3.43 / 3.71; x 9 0.380 / 3.61 / 3.91; 256 x 4 0.356 /
-// 3.36 / 3.67; two blocks, 128 x 5 0.345 / 3.30 / 3.71; x 6 0.362 / 3.37 / 3.82.
-#ifndef PIC_MOVER_PPL
-#define PIC_MOVER_PPL 2
-#endif
-constexpr int kPPL = PIC_MOVER_PPL;
+// A warp's work item is 64 consecutive particles: lane l holds particles 2 l and 2 l + 1 in registers, loaded
+// with one 8-byte load per array.  Capacities are multiples of PIC_CHUNK, so every item lies inside
+// the arrays.  Small CTAs let the register file hold 28 warps of 72 registers.  Measured on B200, ms per
+// pass at 1025^2 (2e7 particles, FP32 deposit) / 4097^2 (2e8) / 4097^2 with the int64 deposit: 128
+// threads x 7 CTAs per SM 0.341 / 3.22 / 3.50; x 6 0.352 / 3.40 / 3.67; x 8 0.361 / 3.43 / 3.71; x 9 0.380 /
+// 3.61 / 3.91; 256 x 4 0.356 / 3.36 / 3.67; items of twice as many particles, 128 x 5 0.345 / 3.30 /
+// 3.71; x 6 0.362 / 3.37 / 3.82.
+constexpr int kPPL = 2;   // particles per lane
 constexpr int kItem = 32 * kPPL;
 
-constexpr int kBlocks = kPPL / 2;
-// Particle k of a lane, relative to the item's first particle plus twice the lane.
-__device__ __forceinline__ constexpr int lane_at(int k) { return 64 * (k >> 1) + (k & 1); }
-
-// The kPPL 4-byte values of one lane, one evict-first 8-byte load / store per block (p: the lane's
-// first).
+// The two 4-byte values of one lane, as one evict-first load / store (p: the lane's first).
 __device__ __forceinline__ void ld_lane(const float* p, float (&a)[kPPL]) {
-#pragma unroll
-  for (int h = 0; h < kBlocks; ++h) {
-    const float2 v = __ldcs(reinterpret_cast<const float2*>(p + 64 * h));
-    a[2 * h] = v.x; a[2 * h + 1] = v.y;
-  }
+  const float2 v = __ldcs(reinterpret_cast<const float2*>(p));
+  a[0] = v.x; a[1] = v.y;
 }
 __device__ __forceinline__ void ld_lane(const uint32_t* p, uint32_t (&a)[kPPL]) {
-#pragma unroll
-  for (int h = 0; h < kBlocks; ++h) {
-    const uint2 v = __ldcs(reinterpret_cast<const uint2*>(p + 64 * h));
-    a[2 * h] = v.x; a[2 * h + 1] = v.y;
-  }
+  const uint2 v = __ldcs(reinterpret_cast<const uint2*>(p));
+  a[0] = v.x; a[1] = v.y;
 }
 __device__ __forceinline__ void st_lane(float* p, const float (&a)[kPPL]) {
-#pragma unroll
-  for (int h = 0; h < kBlocks; ++h) __stcs(reinterpret_cast<float2*>(p + 64 * h), make_float2(a[2 * h], a[2 * h + 1]));
+  __stcs(reinterpret_cast<float2*>(p), make_float2(a[0], a[1]));
 }
 __device__ __forceinline__ void st_lane(uint32_t* p, const uint32_t (&a)[kPPL]) {
-#pragma unroll
-  for (int h = 0; h < kBlocks; ++h) __stcs(reinterpret_cast<uint2*>(p + 64 * h), make_uint2(a[2 * h], a[2 * h + 1]));
+  __stcs(reinterpret_cast<uint2*>(p), make_uint2(a[0], a[1]));
 }
 constexpr int kWarps = PIC_MOVER_THREADS / 32;
 #ifndef PIC_MOVER_MIN_BLOCKS
@@ -265,73 +247,55 @@ __device__ __forceinline__ void cic_i64(long long qf, float fx, float fy, long l
   d = qf - a - b - c;
 }
 
-// Deposit of H blocks of 64 particles, two per lane and block (keys in lane order).  Per block: equal
-// keys of a lane's pair are summed in registers (of two different ones the first goes to rho at
-// once), then the lanes' runs of equal keys are summed over the warp (lane order) and the first lane
-// of each adds the totals to rho.  The blocks' reductions run together.  Called by all lanes.
-template <int H, typename V, typename W>
-__device__ __forceinline__ void lane_deposit(V* rho, int nx, const uint32_t* key, const float* fx, const float* fy,
-                                             W weights) {
+// Deposit of an item's 64 particles, two per lane (keys in lane order): equal keys of a lane's pair are summed
+// in registers (of two different ones the first goes to rho at once), then the lanes' runs of equal
+// keys are summed over the warp (lane order) and the first lane of each adds the totals to rho.
+// Called by all lanes.
+template <typename V, typename W>
+__device__ __forceinline__ void lane_deposit(V* rho, int nx, const uint32_t (&key)[kPPL], const float (&fx)[kPPL],
+                                             const float (&fy)[kPPL], W weights) {
   const int lane = lane_id();
-  V v[H][4];
-  uint32_t rk[H];
-  int end[H];
-  bool head[H];
-  int longest = 0;
+  V v[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0};
+  uint32_t rk = key[0];
+  if (rk != PIC_CELL_OUT) weights(fx[0], fy[0], v[0], v[1], v[2], v[3]);
+  if (key[1] != PIC_CELL_OUT) weights(fx[1], fy[1], b[0], b[1], b[2], b[3]);
+  if (key[1] == rk) {
 #pragma unroll
-  for (int h = 0; h < H; ++h) {
-    V b[4] = {0, 0, 0, 0};
-    v[h][0] = v[h][1] = v[h][2] = v[h][3] = 0;
-    rk[h] = key[2 * h];
-    if (rk[h] != PIC_CELL_OUT) weights(fx[2 * h], fy[2 * h], v[h][0], v[h][1], v[h][2], v[h][3]);
-    if (key[2 * h + 1] != PIC_CELL_OUT) weights(fx[2 * h + 1], fy[2 * h + 1], b[0], b[1], b[2], b[3]);
-    if (key[2 * h + 1] == rk[h]) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) v[h][u] += b[u];
-    } else {
-      if (rk[h] != PIC_CELL_OUT) {
-        V* r = rho + (size_t)cell_j(rk[h]) * nx + cell_i(rk[h]);
-        red_add(r, v[h][0]); red_add(r + 1, v[h][1]); red_add(r + nx, v[h][2]); red_add(r + nx + 1, v[h][3]);
-      }
-      rk[h] = key[2 * h + 1];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) v[h][u] = b[u];
+    for (int u = 0; u < 4; ++u) v[u] += b[u];
+  } else {
+    if (rk != PIC_CELL_OUT) {
+      V* r = rho + (size_t)cell_j(rk) * nx + cell_i(rk);
+      red_add(r, v[0]); red_add(r + 1, v[1]); red_add(r + nx, v[2]); red_add(r + nx + 1, v[3]);
     }
-  }
+    rk = key[1];
 #pragma unroll
-  for (int h = 0; h < H; ++h) {
-    const uint32_t prev = __shfl_up_sync(0xffffffffu, rk[h], 1);
-    head[h] = (lane == 0) || (rk[h] != prev);
-    const unsigned heads = __ballot_sync(0xffffffffu, head[h]);
-    // the lane after this lane's segment, and the segment's length from its head
-    const unsigned after = lane == 31 ? 0u : heads & (0xfffffffeu << lane);
-    const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-    end[h] = after ? __ffs(after) - 1 : 32;
-    longest = max(longest, end[h] - first);
+    for (int u = 0; u < 4; ++u) v[u] = b[u];
   }
-  longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)longest);
+  const uint32_t prev = __shfl_up_sync(0xffffffffu, rk, 1);
+  const bool head = (lane == 0) || (rk != prev);
+  const unsigned heads = __ballot_sync(0xffffffffu, head);
+  // the lane after this lane's segment, and the longest segment of the warp
+  const unsigned after = lane == 31 ? 0u : heads & (0xfffffffeu << lane);
+  const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+  const int end = after ? __ffs(after) - 1 : 32;
+  const int longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)(end - first));
   // only as many shuffle levels as the longest segment needs
   for (int o = 1; o < longest; o <<= 1) {
+    V t[4];
 #pragma unroll
-    for (int h = 0; h < H; ++h) {
-      V t[4];
+    for (int u = 0; u < 4; ++u) t[u] = __shfl_down_sync(0xffffffffu, v[u], o);
+    if (lane + o < end) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) t[u] = __shfl_down_sync(0xffffffffu, v[h][u], o);
-      if (lane + o < end[h]) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) v[h][u] += t[u];
-      }
+      for (int u = 0; u < 4; ++u) v[u] += t[u];
     }
   }
-#pragma unroll
-  for (int h = 0; h < H; ++h)
-    if (head[h] && rk[h] != PIC_CELL_OUT) {
-      V* r = rho + (size_t)cell_j(rk[h]) * nx + cell_i(rk[h]);
-      red_add(r, v[h][0]);
-      red_add(r + 1, v[h][1]);
-      red_add(r + nx, v[h][2]);
-      red_add(r + nx + 1, v[h][3]);
-    }
+  if (head && rk != PIC_CELL_OUT) {
+    V* r = rho + (size_t)cell_j(rk) * nx + cell_i(rk);
+    red_add(r, v[0]);
+    red_add(r + 1, v[1]);
+    red_add(r + nx, v[2]);
+    red_add(r + nx + 1, v[3]);
+  }
 }
 
 // Deferred collision candidates of a warp: cell fx fy vx vy vz pid index, up to one round of
@@ -482,7 +446,7 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
     }
     bool valid[kPPL];
 #pragma unroll
-    for (int k = 0; k < kPPL; ++k) valid[k] = i0 + lane_at(k) < n;
+    for (int k = 0; k < kPPL; ++k) valid[k] = i0 + k < n;
     // ---- pass A: kick and collisions
     if (do_kick) {
       const float2* __restrict__ ef = J.efield;
@@ -572,7 +536,7 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
             cq[1 * kQueue + q] = __float_as_uint(fx[k]); cq[2 * kQueue + q] = __float_as_uint(fy[k]);
             cq[3 * kQueue + q] = __float_as_uint(vx[k]); cq[4 * kQueue + q] = __float_as_uint(vy[k]);
             cq[5 * kQueue + q] = __float_as_uint(vz[k]); cq[6 * kQueue + q] = pid[k];
-            cq[7 * kQueue + q] = (uint32_t)(i0 + lane_at(k));
+            cq[7 * kQueue + q] = (uint32_t)(i0 + k);
             valid[k] = false;   // the queue round finishes this particle
           }
         qn += ncand;
@@ -634,30 +598,25 @@ mover_kernel(const JobDev* __restrict__ jobs, JobState* __restrict__ st, const S
         base = __shfl_sync(0xffffffffu, base, 0);
 #pragma unroll
         for (int k = 0; k < kPPL; ++k)
-          if (valid[k] && absorbed[k]) S.hits[base + hb[k] + __popc(hm[k] & ((1u << lane) - 1u))] = i0 + lane_at(k);
+          if (valid[k] && absorbed[k]) S.hits[base + hb[k] + __popc(hm[k] & ((1u << lane) - 1u))] = i0 + k;
       }
     }
     if (do_dep) {
       if (J.deposit_mode == 0) {
         const float q = S.qdep;
-        lane_deposit<kBlocks, float>(J.rho_f, J.nx, key, fx, fy,
-                                     [q](float x, float y, float& a, float& b, float& cc, float& d) {
-                                       cic_f32(q, x, y, a, b, cc, d);
-                                     });
+        lane_deposit<float>(J.rho_f, J.nx, key, fx, fy,
+                            [q](float x, float y, float& a, float& b, float& cc, float& d) { cic_f32(q, x, y, a, b, cc, d); });
       } else {
-        // block by block: the 64-bit sums of several blocks do not fit the registers
         const long long qf = S.qfix;
-#pragma unroll
-        for (int h = 0; h < kBlocks; ++h)
-          lane_deposit<1, unsigned long long>(
-              reinterpret_cast<unsigned long long*>(J.rho_i), J.nx, key + 2 * h, fx + 2 * h, fy + 2 * h,
-              [qf](float x, float y, unsigned long long& a, unsigned long long& b, unsigned long long& cc,
-                   unsigned long long& d) {
-                long long a_, b_, c_, d_;
-                cic_i64(qf, x, y, a_, b_, c_, d_);
-                a = (unsigned long long)a_; b = (unsigned long long)b_; cc = (unsigned long long)c_;
-                d = (unsigned long long)d_;
-              });
+        lane_deposit<unsigned long long>(
+            reinterpret_cast<unsigned long long*>(J.rho_i), J.nx, key, fx, fy,
+            [qf](float x, float y, unsigned long long& a, unsigned long long& b, unsigned long long& cc,
+                 unsigned long long& d) {
+              long long a_, b_, c_, d_;
+              cic_i64(qf, x, y, a_, b_, c_, d_);
+              a = (unsigned long long)a_; b = (unsigned long long)b_; cc = (unsigned long long)c_;
+              d = (unsigned long long)d_;
+            });
       }
     }
     // ---- stores
