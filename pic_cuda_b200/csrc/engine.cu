@@ -181,36 +181,53 @@ int event_capacity(const pic_job_config& c) {
 // Rows per strip item of a level of the given sides (those of the jobs of a launch), 0 where the tile
 // kernels take the level.  An item is one warp, so a level needs about nine of them per SM to hide their
 // latency chains (twelve on the level-0 up kernel, whose tiles are better at 1025^2), and the largest row
-// count that still gives as many wastes least on the rows a strip recomputes before its first; beyond 72
-// rows the last wave costs more than that saves.  Measured on B200, V-cycle with strips against
+// count that still gives as many wastes least on the rows a strip recomputes before its first, up to
+// 72.  Measured on B200, V-cycle with strips against
 // tiles: 4097^2 277 / 401 us, 2049^2 121 / 139, 1025^2 62.6 / 63.3 (66.9 with the level-0 up as
-// strips too); forced at 513^2 67 / 46.5.  Rows per down item at 4097^2: 14 307 us, 30 301, 46 297,
-// 62 297, 94 300, 190 303; per level-0 up item: 12 338, 24 304, 48 289, 72 285, 96 294.
+// strips too); forced at 513^2 67 / 46.5; in batches, where small levels together reach the line, 64 jobs of
+// 129^2 48 / 48, 300 of 129^2 125 / 157, 16 of 257^2 55.8 / 54.7, 32 of 257^2 75 / 83, 100 of 257^2 155 /
+// 191, 8 of 513^2 82 / 86, 16 of 513^2 118 / 136, 2 of 1025^2 85 / 87, 8 of 1025^2 183 / 228.  Rows per down
+// item at 4097^2: 14 307 us, 30 301, 46 297, 62 297, 94 300, 190 303.
 int64_t strip_items(int n, int leg, int nu, int l, int rows) {
   return (int64_t)(leg == 0 ? mg_down_strips(nu, n) : mg_up_strips(nu, l, n)) * ((n + rows - 1) / rows);
 }
-int strip_rows(int num_sms, const std::vector<int>& sides, int leg, int nu, int l) {
+int64_t strip_items(const std::vector<int>& sides, int leg, int nu, int l, int rows) {
+  int64_t items = 0;
+  for (int n : sides) items += strip_items(n, leg, nu, l, rows);
+  return items;
+}
+int most_strip_rows(int num_sms, const std::vector<int>& sides, int leg, int nu, int l) {
   const int per_sm = leg == 1 && l == 0 ? 12 : 9;
-  for (int rows = mg_strip_rows(leg, nu, l, 72); rows > 0; rows = mg_strip_rows(leg, nu, l, rows - 1)) {
-    int64_t items = 0;
-    for (int n : sides) items += strip_items(n, leg, nu, l, rows);
-    if (items >= (int64_t)per_sm * num_sms) return rows;
-  }
+  for (int rows = mg_strip_rows(leg, nu, l, 72); rows > 0; rows = mg_strip_rows(leg, nu, l, rows - 1))
+    if (strip_items(sides, leg, nu, l, rows) >= (int64_t)per_sm * num_sms) return rows;
   return 0;
 }
-// Rows per strip item of a job's level-0 up leg.  This launch sums the job's residual norm, in an order that
-// follows the items, so the choice looks at the job alone: relres and the cycle a solve stops at must
-// not depend on the jobs beside it.  (Every other leg gives the same bits as tiles and as strips.)
-int up0_rows(int num_sms, int n, int nu) {
-  return nu >= 1 && nu <= kMaxFastNu ? strip_rows(num_sms, {n}, 1, nu, 0) : 0;
+// The level-0 up kernel holds 15 items per SM: where they fill a last wave by less than a third, longer items, as
+// long as there are ten per SM.  Measured on B200, V-cycle at 4097^2 with 54 rows (2.7 waves) 278 us, 72
+// (2.03) 286, 78 (1.9) 272; 32 jobs of 257^2 with 18 rows (1.04) 82.5, 24 (0.8) 75.4; 8 jobs of 513^2 88.9, 82.3.
+int strip_rows(int num_sms, const std::vector<int>& sides, int leg, int nu, int l) {
+  int rows = most_strip_rows(num_sms, sides, leg, nu, l);
+  if (leg != 1 || l != 0) return rows;
+  const int64_t wave = 15ll * num_sms;
+  while (rows > 0 && rows < 96) {
+    const int64_t items = strip_items(sides, leg, nu, l, rows);
+    if (items <= wave || items % wave >= wave / 3) break;
+    const int longer = mg_strip_rows(leg, nu, l, rows + 6);
+    if (longer <= rows || strip_items(sides, leg, nu, l, longer) < 10ll * num_sms) break;
+    rows = longer;
+  }
+  return rows;
 }
 
 // FP64 partial sums of a job's level-0 launches: per init tile r^2, F^2 (pairs) and the charge, or a
-// pair per strip item of the level-0 up kernel.
+// pair per strip item of the level-0 up kernel.  A job has most items in the rows it gets when alone; one
+// that runs as tiles when alone, in the shortest rows.
 int64_t partials_bytes(int num_sms, int n, int nu) {
   const int64_t t = (n + 31) / 32;
-  const int rows = up0_rows(num_sms, n, nu);
-  return std::max<int64_t>(24 * t * t, rows ? 16 * strip_items(n, 1, nu, 0, rows) : 0);
+  int rows = nu >= 1 && nu <= kMaxFastNu ? most_strip_rows(num_sms, {n}, 1, nu, 0) : -1;
+  if (rows == 0)
+    for (int r = mg_strip_rows(1, nu, 0, 72); r > 0; r = mg_strip_rows(1, nu, 0, r - 1)) rows = r;
+  return std::max<int64_t>(24 * t * t, rows > 0 ? 16 * strip_items(n, 1, nu, 0, rows) : 0);
 }
 
 struct Layout {  // byte sizes of one job's device state
@@ -488,7 +505,7 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
       for (int tj = 0; tj < tc; ++tj)
         for (int ti = 0; ti < tc; ++ti) down[l].push_back({id, ti, tj, 0, 1, 0});
       const int tu = (D.nl[l] + 31) / 32;
-      for (int tj = 0; l > 0 && tj < tu; ++tj)
+      for (int tj = 0; tj < tu; ++tj)
         for (int ti = 0; ti < tu; ++ti) up[l].push_back({id, ti, tj, tj * tu + ti, tu * tu, 0});
     }
     if (E->cluster_C > 0 && D.nl[D.lc] > PIC_COARSE_MAX) {   // above one CTA's shared memory
@@ -503,40 +520,29 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   // the count every job has, where kernels with compile-time shapes exist for it (the maxima start at 1)
   const int fast_pre = nu_pre_min == nu_pre_max && nu_pre_max <= kMaxFastNu ? nu_pre_max : -1;
   const int fast_post = nu_post_min == nu_post_max && nu_post_max <= kMaxFastNu ? nu_post_max : -1;
-  // strips of the level-0 up leg (by post-sweeps): job by job; the other jobs' tiles stay
-  std::vector<TileRef> sdown[PIC_MAX_LEVELS], sup[PIC_MAX_LEVELS], sup0[kMaxFastNu + 1];
-  auto add_items = [&](std::vector<TileRef>& v, int id, int leg, int nu, int l, int rows) {
-    const int n = E->jobs[id].dev.nl[l];
-    const int ts = leg == 0 ? mg_down_strips(nu, n) : mg_up_strips(nu, l, n), tr = (n + rows - 1) / rows;
-    for (int tj = 0; tj < tr; ++tj)
-      for (int ti = 0; ti < ts; ++ti) v.push_back({id, ti, tj, tj * ts + ti, rows, 0});
-    return tr * ts;
-  };
-  for (int id : ids) {
-    const JobDev& D = E->jobs[id].dev;
-    if (D.lc == 0) continue;
-    const int n = D.nl[0], rows = up0_rows(E->num_sms, n, D.nu_post), tu = (n + 31) / 32;
-    if (rows) {
-      finish.push_back(id);
-      finish.push_back(add_items(sup0[D.nu_post], id, 1, D.nu_post, 0, rows));
-      continue;
-    }
-    for (int tj = 0; tj < tu; ++tj)
-      for (int ti = 0; ti < tu; ++ti) up[0].push_back({id, ti, tj, tj * tu + ti, tu * tu, 0});
-    if (fast_post >= 0) { finish.push_back(id); finish.push_back(tu * tu); }
-  }
-  // strips of the other legs: where the level has enough items over all jobs
+  std::vector<TileRef> sdown[PIC_MAX_LEVELS], sup[PIC_MAX_LEVELS];
   for (int l = 0; l < max_depth; ++l)
     for (int leg = 0; leg < 2; ++leg) {
       const int nu = leg == 0 ? fast_pre : fast_post;
-      if (nu < 0 || (leg == 1 && l == 0)) continue;
+      if (nu < 0) continue;
       std::vector<int> sides;
       for (int id : ids)
         if (l < E->jobs[id].dev.lc) sides.push_back(E->jobs[id].dev.nl[l]);
       const int rows = strip_rows(E->num_sms, sides, leg, nu, l);
-      if (!rows) continue;
-      for (int id : ids)
-        if (l < E->jobs[id].dev.lc) add_items((leg == 0 ? sdown : sup)[l], id, leg, nu, l, rows);
+      for (int id : ids) {
+        const JobDev& D = E->jobs[id].dev;
+        if (l >= D.lc) continue;
+        const int n = D.nl[l], tu = (n + 31) / 32;
+        int parts = tu * tu;   // tile kernels
+        if (rows) {
+          const int ts = leg == 0 ? mg_down_strips(nu, n) : mg_up_strips(nu, l, n), tr = (n + rows - 1) / rows;
+          for (int tj = 0; tj < tr; ++tj)
+            for (int ti = 0; ti < ts; ++ti)
+              (leg == 0 ? sdown : sup)[l].push_back({id, ti, tj, tj * ts + ti, rows, 0});
+          parts = tr * ts;
+        }
+        if (l == 0 && leg == 1) { finish.push_back(id); finish.push_back(parts); }
+      }
     }
   std::vector<TileRef> all;
   size_t off_init = all.size(); all.insert(all.end(), init.begin(), init.end());
@@ -547,8 +553,6 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
   size_t off_sd[PIC_MAX_LEVELS], off_su[PIC_MAX_LEVELS];
   for (int l = 0; l < PIC_MAX_LEVELS; ++l) { off_sd[l] = all.size(); all.insert(all.end(), sdown[l].begin(), sdown[l].end()); }
   for (int l = 0; l < PIC_MAX_LEVELS; ++l) { off_su[l] = all.size(); all.insert(all.end(), sup[l].begin(), sup[l].end()); }
-  size_t off_s0[kMaxFastNu + 1];
-  for (int nu = 0; nu <= kMaxFastNu; ++nu) { off_s0[nu] = all.size(); all.insert(all.end(), sup0[nu].begin(), sup0[nu].end()); }
   if (!all.empty()) {
     CK(cudaMalloc(&out.d_tiles, all.size() * sizeof(TileRef)));
     CK(cudaMemcpy(out.d_tiles, all.data(), all.size() * sizeof(TileRef), cudaMemcpyHostToDevice));
@@ -571,7 +575,6 @@ int build_mg(pic_engine* E, const std::vector<int>& ids, MgBuild& out) {
     M.down_items[l] = out.d_tiles + off_sd[l]; M.n_down_items[l] = (int)sdown[l].size();
     M.up_items[l] = out.d_tiles + off_su[l]; M.n_up_items[l] = (int)sup[l].size();
   }
-  for (int nu = 0; nu <= kMaxFastNu; ++nu) { M.up0_items[nu] = out.d_tiles + off_s0[nu]; M.n_up0_items[nu] = (int)sup0[nu].size(); }
   M.coarse_jobs = out.d_coarse; M.n_coarse = (int)coarse.size();
   M.cluster_jobs = out.d_coarse + coarse.size(); M.n_cluster = (int)cluster.size();
   M.finish_jobs = out.d_coarse + coarse.size() + cluster.size(); M.n_finish = (int)finish.size() / 2;

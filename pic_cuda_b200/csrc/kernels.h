@@ -86,11 +86,8 @@ struct MgLaunch {
   const int* cluster_jobs; int n_cluster;                // thread-block-cluster coarse solve
   // strip items (mg_strips.cuh) per level, empty where the tile kernels take it
   const TileRef* down_items[PIC_MAX_LEVELS]; int n_down_items[PIC_MAX_LEVELS];
-  const TileRef* up_items[PIC_MAX_LEVELS]; int n_up_items[PIC_MAX_LEVELS];   // levels >= 1
-  // level 0's up leg: strip items of the jobs large enough for them, by post-sweeps; up_tiles[0] holds
-  // the other jobs' tiles
-  const TileRef* up0_items[kMaxFastNu + 1]; int n_up0_items[kMaxFastNu + 1];
-  const int* finish_jobs; int n_finish;                  // (job, level-0 partials) where mg_finish_kernel ends the cycle
+  const TileRef* up_items[PIC_MAX_LEVELS]; int n_up_items[PIC_MAX_LEVELS];
+  const int* finish_jobs; int n_finish;                  // (job, level-0 partials) of the jobs with lc >= 1
   int cluster_C;
   size_t cluster_smem;
   int max_depth;                                         // max lc over jobs

@@ -23,11 +23,13 @@
 #pragma once
 #include "common.cuh"
 #include "kernels.h"
+#include "mg_norm.cuh"
 #include "tma.cuh"
 
 namespace mgs {
 
 constexpr int kWarps = 4;                 // strips per CTA
+constexpr int up_warps(int mode) { return mode ? 3 : kWarps; }   // the same of the up kernel
 
 // Owned lanes [lo, lo + lanes) of a strip and its owned columns, for the down leg (residual and
 // full weighting after the sweeps), the up leg and the up leg of level 0 (FP64 residual after
@@ -283,7 +285,7 @@ struct __align__(16) UpStep {
 };
 
 template <int NU, int MODE, bool EDGE>
-__device__ __forceinline__ double up_strip(const UpArgs& A, UpStep<MODE>* ring) {
+__device__ __forceinline__ void up_strip(const UpArgs& A, UpStep<MODE>* ring, mgn::Sum& norm) {
   constexpr int T = 2 * NU, WIN = T + 1, WF = T, LO = up_lo(NU, MODE), LANES = up_lanes(NU, MODE), D = up_ring(MODE);
   const int lane = threadIdx.x & 31;
   const int n = A.n, c0 = A.c0, pf = A.pf;
@@ -342,7 +344,6 @@ __device__ __forceinline__ double up_strip(const UpArgs& A, UpStep<MODE>* ring) 
 #pragma unroll
   for (int a = 0; a < WF; ++a) F[a][0] = F[a][1] = 0.f;
   P[0][0] = P[0][1] = P[1][0] = P[1][1] = 0.0;
-  double ar = 0.0;
   // the coarse row of the first step's row goes through the ring's last slot
   request_c(ring[D - 1], js >> 1);
   tma::cp_async_commit();
@@ -435,9 +436,7 @@ __device__ __forceinline__ double up_strip(const UpArgs& A, UpStep<MODE>* ring) 
         store2(out, (float)d0, (float)d1, own && colin1);
         if (EDGE) store1(out, (float)d0, own && !colin1);
         pout += n;
-        const double s0 = own ? d0 : 0.0, s1 = own ? d1 : 0.0;
-        ar += s0 * s0;
-        ar += s1 * s1;
+        norm.add(own ? mgn::pair_of(d0, d1) : 0.0);
       }
       out += pf;
     }
@@ -448,17 +447,18 @@ __device__ __forceinline__ double up_strip(const UpArgs& A, UpStep<MODE>* ring) 
     if (MODE) { P[0][0] = P[D][0]; P[0][1] = P[D][1]; P[1][0] = P[D + 1][0]; P[1][1] = P[D + 1][1]; }
   }
   tma::cp_async_wait<0>();
-  return ar;
 }
 
+// Level 0: 15 warps per SM at 128 registers (five CTAs of three warps; with four of four the norm's sums
+// spill more: V-cycle at 2049^2 116.1 us against 114.2, 4097^2 274.8 against 272).
 template <int NU, int MODE>
-__global__ void __launch_bounds__(32 * kWarps, MODE ? 4 : 5) mg_up_strip_kernel(const TileRef* __restrict__ items, int n_items,
+__global__ void __launch_bounds__(32 * up_warps(MODE), 5) mg_up_strip_kernel(const TileRef* __restrict__ items, int n_items,
                                                                   const JobDev* __restrict__ jobs,
                                                                   JobState* __restrict__ st, int l) {
-  __shared__ __align__(16) UpStep<MODE> ring[kWarps][up_ring(MODE)];
+  __shared__ __align__(16) UpStep<MODE> ring[up_warps(MODE)][up_ring(MODE)];
   constexpr int T = 2 * NU;
   tma::pdl_trigger();
-  const int warp = threadIdx.x >> 5, item = blockIdx.x * kWarps + warp, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, item = blockIdx.x * up_warps(MODE) + warp, lane = threadIdx.x & 31;
   if (item >= n_items) return;
   // the job state changes only in mg_finish_kernel, at the end of a V-cycle (the next V-cycle's
   // first launch waits for it), so it is read before waiting for the previous launch
@@ -489,15 +489,16 @@ __global__ void __launch_bounds__(32 * kWarps, MODE ? 4 : 5) mg_up_strip_kernel(
     A.inv_h2 = 1.0 / (J.h * J.h);
     A.rhs_scale = J.rhs_scale;
   }
+  const double rnorm2 = MODE ? S.rnorm2 : 0.0;
   tma::pdl_wait();
   const bool edge = x0 < 1 || x0 + 63 > A.n - 2 || A.r0 - (MODE ? 2 * T + 3 : T + 1) < 0 || A.r1 + T + 9 > A.n - 1;
-  double ar;
-  if (edge) ar = up_strip<NU, MODE, true>(A, ring[warp]);
-  else ar = up_strip<NU, MODE, false>(A, ring[warp]);
+  const mgn::Scale scale(rnorm2, A.n);
+  mgn::Sum norm(scale);
+  if (edge) up_strip<NU, MODE, true>(A, ring[warp], norm);
+  else up_strip<NU, MODE, false>(A, ring[warp], norm);
   if (MODE) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) ar += __shfl_xor_sync(0xffffffffu, ar, o);
-    if (lane == 0) J.partials[2 * (tr.pbase + tr.local)] = ar;
+    const mgn::Part p = mgn::warp_part(norm.part(scale, rows));
+    if (lane == 0) reinterpret_cast<mgn::Part*>(J.partials)[tr.pbase + tr.local] = p;
   }
 }
 

@@ -23,13 +23,14 @@
 //   (opt-in: levels up to 257^2 or 513^2 in one thread-block cluster, mg_cluster.cu)
 //   mg_up      prolongation + nu_post sweeps on 32x32 tiles; on level 0 also the FP64
 //              update phi += e, the new FP64 residual and the tile's partial norm;
-//              mg_finish (one CTA per job) sums the partials in a fixed order
+//              mg_finish (one CTA per job) adds the partials (mg_norm.cuh: no order matters)
 //              (deterministic), counts the cycle and decides convergence.  The generic
 //              kernels (mixed smoothing counts) still let the last tile CTA of a job do it.
 #include <algorithm>
 #include "common.cuh"
 #include "kernels.h"
 #include "mg_coarse.cuh"
+#include "mg_norm.cuh"
 #include "mg_strips.cuh"
 #include "mg_tiles.h"
 #include "tma.cuh"
@@ -716,7 +717,7 @@ __global__ void __launch_bounds__(256) mg_up_kernel(const TileRef* __restrict__ 
   const RhoSrc rho{J.deposit_mode, J.rho_f, J.rho_i, J.rho_d};
   float* const f0 = fsel ? J.f[0] : J.f0b;   // the new defect goes to the other buffer
   double* const partials = J.partials;
-  const double tol = J.tol;
+  const double tol = J.tol, rnorm2 = T.rnorm2;
   const int max_cycles = J.max_cycles;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 2
@@ -768,29 +769,35 @@ __global__ void __launch_bounds__(256) mg_up_kernel(const TileRef* __restrict__ 
       P[py * PW + px] = v;
     }
   __syncthreads();
-  double ar = 0.0;
-  for (int oy = warp; oy < kTU; oy += 8) {
-    const int ox = lane;
+  const mgn::Scale scale(rnorm2, nf);
+  mgn::Sum norm(scale);
+  double r_own[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int ox = lane, oy = 4 * warp + u;
     const int gx = i0 + ox, gy = j0 + oy;
-    if (gx >= nf || gy >= nf) continue;
-    const size_t g = (size_t)gy * nf + gx;
-    const int q = (oy + 1) * PW + (ox + 1);
-    const double rv = rho[g];
     double r = 0.0;
-    if (gx > 0 && gx < nf - 1 && gy > 0 && gy < nf - 1) {
-      const double lap = P[q - PW] + P[q + PW] + P[q - 1] + P[q + 1] - 4.0 * P[q];
-      // mode 1: as in the kernels with compile-time shapes, one of which a job gets when it is alone
-      r = mode == 1 ? mgs::defect(lap, inv_h2, rhs_scale, rv, gy) : rhs_scale * rv - lap * inv_h2;
+    if (gx < nf && gy < nf) {
+      const size_t g = (size_t)gy * nf + gx;
+      const int q = (oy + 1) * PW + (ox + 1);
+      const double rv = rho[g];
+      if (gx > 0 && gx < nf - 1 && gy > 0 && gy < nf - 1) {
+        const double lap = P[q - PW] + P[q + PW] + P[q - 1] + P[q + 1] - 4.0 * P[q];
+        // mode 1: as in the kernels with compile-time shapes, one of which a job gets when it is alone
+        r = mode == 1 ? mgs::defect(lap, inv_h2, rhs_scale, rv, gy) : rhs_scale * rv - lap * inv_h2;
+      }
+      pn[g] = P[q];
+      f0[(size_t)gy * pf + gx] = (float)r;
     }
-    pn[g] = P[q];
-    f0[(size_t)gy * pf + gx] = (float)r;
-    ar += r * r;
+    r_own[u] = r;
   }
-  const double sr = block_sum(ar);
-  if (threadIdx.x == 0) partials[2 * (tr.pbase + tr.local)] = sr;
+  mgn::add_rows4(norm, r_own);
+  __shared__ mgn::Part ws[2][8];
+  const mgn::Part part = mgn::cta_part(norm.part(scale, 2), ws[0]);
+  if (threadIdx.x == 0) reinterpret_cast<mgn::Part*>(partials)[tr.pbase + tr.local] = part;
   if (last_of_job(T, tr.nlocal)) {
     __threadfence();
-    const double r2 = ordered_sum(partials + 2 * tr.pbase, tr.nlocal, 2, 0);
+    const double r2 = mgn::total(mgn::sum_partials(partials + 2 * tr.pbase, tr.nlocal, ws[1]), scale);
     if (threadIdx.x != 0) return;
     T.rnorm2 = r2;
     T.relres = T.fnorm2 > 0.0 ? sqrt(r2 / T.fnorm2) : sqrt(r2);
@@ -1008,6 +1015,7 @@ __global__ void __launch_bounds__(NT, MODE == 0 ? 1 : NT == 256 ? 5 : 2)
   const RhoSrc rho{J.deposit_mode, J.rho_f, J.rho_i, J.rho_d};
   float* const f0 = fsel ? J.f[0] : J.f0b;   // the new defect goes to the other buffer
   double* const partials = J.partials;
+  const double rnorm2 = T.rnorm2;
   const int t = threadIdx.x;
   if (t == 0) {
     tma::mbar_init(&mbar, 1);
@@ -1090,49 +1098,55 @@ __global__ void __launch_bounds__(NT, MODE == 0 ? 1 : NT == 256 ? 5 : 2)
       }
     }
     __syncthreads();
-    double ar = 0.0, r_own = 0.0;
+    // thread t: column t & 31 of rows 4 (t >> 5) .. + 3 (256 threads), or the one node t (1024)
+    const mgn::Scale scale(rnorm2, nf);
+    mgn::Sum norm(scale);
+    double r_own[NO];
 #pragma unroll
     for (int u = 0; u < NO; ++u) {
-      const int k = t + u * NT;
+      const int k = NO == 1 ? t : 128 * (t >> 5) + 32 * u + (t & 31);
       const int ox = k & 31, oy = k >> 5;
       const int gx = i0 + ox, gy = j0 + oy;
-      if (gx >= nf || gy >= nf) continue;
-      const int g = gy * nf + gx;
-      const int q = (oy + 1) * PW + (ox + 1);
-      const double rv = rho.mode == 0 ? (double)reinterpret_cast<const float*>(RH)[k]
-                        : rho.mode == 1 ? (double)reinterpret_cast<const long long*>(RH)[k] * 0x1p-40 : RH[k];
       double r = 0.0;
-      if (gx > 0 && gx < nf - 1 && gy > 0 && gy < nf - 1) {
-        const double lap = P64[q - PW] + P64[q + PW] + P64[q - 1] + P64[q + 1] - 4.0 * P64[q];
-        r = mgs::defect(lap, inv_h2, rhs_scale, rv, gy);
+      if (gx < nf && gy < nf) {
+        const int g = gy * nf + gx;
+        const int q = (oy + 1) * PW + (ox + 1);
+        const double rv = rho.mode == 0 ? (double)reinterpret_cast<const float*>(RH)[k]
+                          : rho.mode == 1 ? (double)reinterpret_cast<const long long*>(RH)[k] * 0x1p-40 : RH[k];
+        if (gx > 0 && gx < nf - 1 && gy > 0 && gy < nf - 1) {
+          const double lap = P64[q - PW] + P64[q + PW] + P64[q - 1] + P64[q + 1] - 4.0 * P64[q];
+          r = mgs::defect(lap, inv_h2, rhs_scale, rv, gy);
+        }
+        pn[g] = P64[q];
+        f0[gy * pf + gx] = (float)r;
       }
-      pn[g] = P64[q];
-      f0[gy * pf + gx] = (float)r;
-      if constexpr (NT == 256) ar += r * r;
-      else r_own = r;
+      r_own[u] = r;
     }
-    if constexpr (NT != 256) {   // the order of additions of 256 threads with four nodes each
+    if constexpr (NT == 256) {
+      mgn::add_rows4(norm, r_own);
+    } else {
       static_assert(NO == 1, "one owned node per thread");
       __syncthreads();           // rho in RH has been read
-      RH[t] = r_own;
+      RH[t] = r_own[0];
       __syncthreads();
-      if (t < 256)
+      if (t < 256) {
+        double r4[4];
 #pragma unroll
-        for (int u = 0; u < kTU * kTU / 256; ++u) {
-          const double r = RH[t + 256 * u];
-          ar += r * r;
-        }
+        for (int u = 0; u < 4; ++u) r4[u] = RH[128 * (t >> 5) + 32 * u + (t & 31)];
+        mgn::add_rows4(norm, r4);
+      }
     }
     // the tile's partial only: the job's norm, convergence test and buffer swap follow in
     // mg_finish_kernel, so no CTA waits for its stores or a shared ticket before it leaves
-    const double sr = block_sum(ar);
-    if (t == 0) partials[2 * (tr.pbase + tr.local)] = sr;
+    __shared__ mgn::Part ws[NT / 32];
+    const mgn::Part part = mgn::cta_part(norm.part(scale, 2), ws);
+    if (t == 0) reinterpret_cast<mgn::Part*>(partials)[tr.pbase + tr.local] = part;
   }
 }
 
 // End of a V-cycle for the jobs whose level 0 ran in mg_up_fast_kernel<., 1, .> or
 // mg_up_strip_kernel<., 1>: one
-// 1024-thread CTA per job sums their partial norms in a fixed order, counts the cycle,
+// 1024-thread CTA per job sums their partial norms (mg_norm.cuh), counts the cycle,
 // swaps the potential and defect buffers and takes a converged job out of the running count.  Launched after the
 // level-0 up kernel (waits for it in tma::pdl_wait); the next V-cycle's first launch waits for
 // this one.
@@ -1152,9 +1166,11 @@ __global__ void __launch_bounds__(1024) mg_finish_kernel(const int* __restrict__
   const int job = job_list[2 * blockIdx.x], n = job_list[2 * blockIdx.x + 1];
   const JobDev& J = jobs[job];
   JobState& T = st[job];
+  __shared__ mgn::Part ws[32];
   if (!T.converged) {
-    const double r2 = ordered_sum(J.partials, n, 2, 0);
+    const mgn::Part sum = mgn::sum_partials(J.partials, n, ws);
     if (threadIdx.x == 0) {
+      const double r2 = mgn::total(sum, mgn::Scale(T.rnorm2, J.nx));
       T.rnorm2 = r2;
       T.relres = T.fnorm2 > 0.0 ? sqrt(r2 / T.fnorm2) : sqrt(r2);
       T.cycles += 1;
@@ -1235,9 +1251,9 @@ void down_strips(int n_items, const TileRef* items, bool pdl, const EngineLaunch
 }
 template <int NU>
 void up_strips(int n_items, const TileRef* items, bool pdl, const EngineLaunch& L, int l, cudaStream_t s) {
-  const int grid = (n_items + mgs::kWarps - 1) / mgs::kWarps;
-  if (l == 0) launch_k(mgs::mg_up_strip_kernel<NU, 1>, grid, 32 * mgs::kWarps, 0, pdl, s, items, n_items, L.jobs, L.st, l);
-  else launch_k(mgs::mg_up_strip_kernel<NU, 0>, grid, 32 * mgs::kWarps, 0, pdl, s, items, n_items, L.jobs, L.st, l);
+  const int w = mgs::up_warps(l == 0 ? 1 : 0), grid = (n_items + w - 1) / w;
+  if (l == 0) launch_k(mgs::mg_up_strip_kernel<NU, 1>, grid, 32 * w, 0, pdl, s, items, n_items, L.jobs, L.st, l);
+  else launch_k(mgs::mg_up_strip_kernel<NU, 0>, grid, 32 * w, 0, pdl, s, items, n_items, L.jobs, L.st, l);
 }
 
 // ---------------------------------------------------------------- levels 1 .. lc in one launch
@@ -1354,8 +1370,8 @@ int mg_strip_rows(int leg, int nu, int level, int at_most) { return mgs::rows_fi
 // Launch of one level.  When every job of the launch has the same smoothing count (1 .. kMaxFastNu):
 // the strip kernels where the level has enough items for them (strip_rows in engine.cu), else the
 // compile-time-shape tile kernels, on 1024-thread CTAs where a level has at most wide_factor
-// (default 2) tiles per SM.  Otherwise the generic tile kernels.  Level 0's up leg sums the residual norm
-// and chooses strips job by job (build_mg in engine.cu).  pdl: the launch follows a kernel
+// (default 2) tiles per SM.  Otherwise the generic tile kernels.  Every choice gives the same bits, the
+// residual norm included.  pdl: the launch follows a kernel
 // of the V-cycle that this one's prologue may overlap (programmatic serialisation).
 static bool launch_down(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, cudaStream_t s) {
   if (M.n_down_items[l]) {
@@ -1372,60 +1388,36 @@ static bool launch_down(const MgLaunch& M, int l, const EngineLaunch& L, bool pd
   mg_down_kernel<<<M.n_down[l], 256, down_smem(M.nu_pre_max), s>>>(M.down_tiles[l], L.jobs, L.st, l);
   return false;
 }
-using StripLaunch = void (*)(int, const TileRef*, bool, const EngineLaunch&, int, cudaStream_t);
-static StripLaunch up_strips_of(int nu) {
-  return nu == 1 ? up_strips<1> : nu == 2 ? up_strips<2> : nu == 3 ? up_strips<3> : up_strips<4>;
-}
-static bool has_up(const MgLaunch& M, int l) {
-  bool any = M.n_up[l] || M.n_up_items[l];
-  if (l == 0)
-    for (int n : M.n_up0_items) any |= n != 0;
-  return any;
-}
-// Does mg_finish_kernel end the V-cycle of every job?
-static bool all_finish(const MgLaunch& M) {
-  return M.n_finish && !M.n_upd && !(M.n_up[0] && M.fast_nu_post < 0);
-}
-static bool launch_up(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, const VcycleLoop* cond, cudaStream_t s,
-                      int& k) {
-  if (l == 0)
-    for (int nu = 1; nu <= kMaxFastNu; ++nu)
-      if (M.n_up0_items[nu]) {
-        up_strips_of(nu)(M.n_up0_items[nu], M.up0_items[nu], pdl && M.pdl, L, 0, s);
-        pdl = true;
-        ++k;
-      }
-  if (M.n_up_items[l]) {
-    up_strips_of(M.fast_nu_post)(M.n_up_items[l], M.up_items[l], pdl && M.pdl, L, l, s);
-    pdl = true;
-    ++k;
-  } else if (M.n_up[l] && M.fast_nu_post >= 0) {
-    up_fast(M.fast_nu_post, M.n_up[l], M.n_up[l] <= M.wide_factor * L.num_sms, pdl && M.pdl, M.up_tiles[l], L.jobs,
-            L.st, l, l == 0 ? 1 : 0, s);
-    pdl = true;
-    ++k;
-  } else if (M.n_up[l]) {
+static bool launch_up(const MgLaunch& M, int l, const EngineLaunch& L, bool pdl, const VcycleLoop* cond, cudaStream_t s) {
+  if (M.fast_nu_post < 0) {
     mg_up_kernel<<<M.n_up[l], 256, up_smem(M.nu_post_max), s>>>(M.up_tiles[l], L.jobs, L.st, l, l == 0 ? 1 : 0,
                                                                 L.running);
-    pdl = false;
-    ++k;
+    return false;
   }
-  if (l == 0 && M.n_finish) {
-    launch_k(mg_finish_kernel, M.n_finish, 1024, 0, pdl && M.pdl, s, M.finish_jobs, L.jobs, L.st, L.running,
-             cond && all_finish(M) ? *cond : VcycleLoop{});
-    ++k;
+  if (M.n_up_items[l]) {
+    auto* f = M.fast_nu_post == 1 ? up_strips<1> : M.fast_nu_post == 2 ? up_strips<2> : M.fast_nu_post == 3 ? up_strips<3>
+                                                                                                          : up_strips<4>;
+    f(M.n_up_items[l], M.up_items[l], pdl && M.pdl, L, l, s);
+  } else {
+    up_fast(M.fast_nu_post, M.n_up[l], M.n_up[l] <= M.wide_factor * L.num_sms, pdl && M.pdl, M.up_tiles[l], L.jobs,
+            L.st, l, l == 0 ? 1 : 0, s);
   }
-  return pdl;
+  if (l == 0)
+    launch_k(mg_finish_kernel, M.n_finish, 1024, 0, M.pdl != 0, s, M.finish_jobs, L.jobs, L.st, L.running,
+             cond ? *cond : VcycleLoop{});
+  return true;
 }
 
 int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, const VcycleLoop* cond, cudaStream_t s) {
   int k = 0;
   // the loop's condition in the last kernel where that is mg_finish_kernel, else after it
+  const bool fused = M.n_up[0] && M.fast_nu_post >= 0 && !M.n_upd;
   auto end_loop = [&]() {
-    if (!cond || all_finish(M)) return;
+    if (!cond || fused) return;
     vcycle_condition_kernel<<<1, 1, 0, s>>>(L.running, *cond);
     ++k;
   };
+  const VcycleLoop* const up_cond = fused ? cond : nullptr;
   if (M.levels_grid > 0 && M.max_depth >= 2 && !M.n_cluster) {
     if (M.n_down[0]) { launch_down(M, 0, L, false, s); ++k; }
     MgLevelsArgs a{};
@@ -1450,7 +1442,7 @@ int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, const VcycleLoop*
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, mg_levels_kernel, a);
     ++k;
-    if (has_up(M, 0)) launch_up(M, 0, L, false, cond, s, k);
+    if (M.n_up[0]) k += launch_up(M, 0, L, false, up_cond, s) ? 2 : 1;   // + mg_finish_kernel
     if (M.n_upd) { mg_up_kernel<<<M.n_upd, 256, up_smem(0), s>>>(M.upd_tiles, L.jobs, L.st, 0, 2, L.running); ++k; }
     end_loop();
     return k;
@@ -1472,7 +1464,7 @@ int launch_mg_vcycle(const EngineLaunch& L, const MgLaunch& M, const VcycleLoop*
   }
   if (M.n_cluster) { k += launch_mg_cluster(M.cluster_jobs, M.n_cluster, M.cluster_C, M.cluster_smem, L.jobs, L.st, s); prev_fast = false; }
   for (int l = M.max_depth - 1; l >= 0; --l)
-    if (has_up(M, l)) prev_fast = launch_up(M, l, L, prev_fast, cond, s, k);
+    if (M.n_up[l]) { prev_fast = launch_up(M, l, L, prev_fast, up_cond, s); k += (prev_fast && l == 0) ? 2 : 1; }
   if (M.n_upd) { mg_up_kernel<<<M.n_upd, 256, up_smem(0), s>>>(M.upd_tiles, L.jobs, L.st, 0, 2, L.running); ++k; }
   end_loop();
   return k;

@@ -56,3 +56,25 @@ def test_norm_does_not_depend_on_the_batch(jobs):
 ], ids=["tiles", "tiles_and_strips"])
 def test_mixed_post_smoothing_keeps_each_result(jobs):
     test_norm_does_not_depend_on_the_batch(jobs)
+
+
+# every kernel that sums the norm: the one-CTA solver's update, 1024- and 256-thread tiles, strips and the
+# general kernel.  Tolerance: the residual's own rounding, a few ulp of phi / h^2 per node, and 1e-13 for the sums.
+@pytest.mark.parametrize("n", [3, 33, 65, 129, 257, 1025, 2049])
+@pytest.mark.parametrize("nu", [1, 2, 4, 5])
+def test_norm_equals_the_residual_of_phi(n, nu):
+    import torch
+    from pic_cuda_b200.engine import solve_multigrid_f64
+    h = 0.3 / (n - 1)
+    rho = torch.randn((n, n), dtype=torch.float64, generator=torch.Generator().manual_seed(n)).cuda()
+    for cycles in (1, 3):
+        phi = torch.zeros_like(rho)
+        _, rel, _ = solve_multigrid_f64(phi, rho, n, n, 0, h, 1.15, nu, nu, 2, 0.0, cycles)
+        p, f = phi.cpu().numpy().astype(np.longdouble), rho.cpu().numpy().astype(np.longdouble)
+        r = f[1:-1, 1:-1] - (p[:-2, 1:-1] + p[2:, 1:-1] + p[1:-1, :-2] + p[1:-1, 2:] - 4 * p[1:-1, 1:-1]) / (
+            np.longdouble(h) * np.longdouble(h))
+        rnorm, fnorm = np.sqrt((r * r).sum()), np.sqrt((f * f).sum())
+        tol = 1e-13 + 16 * 2.0 ** -53 * n * float(np.abs(p).max() / h / h / rnorm)
+        assert abs(rel / float(rnorm / fnorm) - 1) < tol
+    zero = torch.zeros_like(rho)
+    assert solve_multigrid_f64(zero.clone(), zero, n, n, 0, h, 1.15, nu, nu, 2, 0.0, 2)[1] == 0.0
