@@ -70,28 +70,31 @@ __device__ __forceinline__ double total(const Part& p, const Scale& s) {
 // Squares of a pair's residuals, added.
 __device__ __forceinline__ double pair_of(double r0, double r1) { return __dadd_rn(__dmul_rn(r0, r0), __dmul_rn(r1, r1)); }
 
-// Sum over the warp.
+// Sum over the warp (over its first LANES lanes, in those).
+template <int LANES = 32>
 __device__ __forceinline__ Part warp_part(Part p) {
 #pragma unroll
-  for (int o = 16; o; o >>= 1)
+  for (int o = LANES / 2; o; o >>= 1)
     p.add(Part{__shfl_xor_sync(0xffffffffu, p.first, o), __shfl_xor_sync(0xffffffffu, p.second, o)});
   return p;
 }
-// Sum over the CTA, in the threads of the first warp (ws: one entry per warp).
-__device__ __forceinline__ Part cta_part(Part p, Part* ws) {
+// Sum over a CTA of WARPS warps, in its first thread.
+template <int WARPS>
+__device__ __forceinline__ Part cta_part(Part p, Part (&ws)[WARPS]) {
   p = warp_part(p);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) ws[warp] = p;
   __syncthreads();
-  if (warp == 0) p = warp_part(lane < (int)(blockDim.x >> 5) ? ws[lane] : Part{0.0, 0});
+  if (warp == 0) p = warp_part<WARPS>(ws[lane & (WARPS - 1)]);
   return p;
 }
-// Sum of n partials by the whole CTA; valid in the first warp.  Eight loads of a thread are issued ahead of the
+// Sum of n partials by a CTA of WARPS warps, in its first thread.  Eight loads of a thread are issued ahead of the
 // additions (16.4k partials at 4097^2 as tiles).
-__device__ __forceinline__ Part sum_partials(const double* partials, int n, Part* ws) {
+template <int WARPS>
+__device__ __forceinline__ Part sum_partials(const double* partials, int n, Part (&ws)[WARPS]) {
   Part p{0.0, 0};
 #pragma unroll 8
-  for (int k = threadIdx.x; k < n; k += blockDim.x) p.add(reinterpret_cast<const Part*>(partials)[k]);
+  for (int k = threadIdx.x; k < n; k += 32 * WARPS) p.add(reinterpret_cast<const Part*>(partials)[k]);
   return cta_part(p, ws);
 }
 
