@@ -31,3 +31,25 @@ def test_wide_level0_tiles_same_bits(nx, deposit, nu):
     assert out[0][2] >= 1
     assert out[0][1:] == out[1][1:]
     assert np.array_equal(out[0][0], out[1][0])
+
+
+# 65^2 with the one-CTA solver from 33^2 down, so that its level 0 has tiles
+@pytest.mark.parametrize("nu", [1, 2, 3, 4])
+def test_wide_level0_tiles_of_the_smallest_grid(nu):
+    rho = np.random.default_rng(nu).standard_normal((65, 65)) * 1e-6
+    out = []
+    for wide in (0, 64):
+        e = Engine(0)
+        e.set_option(L.OPT_MG_COARSE_TOP, 33)
+        e.set_option(L.OPT_MG_WIDE_TILES, wide)
+        cfg = cf.plasma(65, 0.01, 1000, deposit=L.DEPOSIT_I64, seed=3, tol=1e-6)
+        cfg.nu_pre = cfg.nu_post = nu
+        cfg.max_cycles = 6
+        j = e.add_job(cfg)
+        j.set_grid(L.GRID_RHO, rho)
+        j.solve_field()
+        d = j.diagnostics()
+        out.append((j.get_grid(L.GRID_PHI), d["relres"], d["vcycles"]))
+        e.close()
+    assert out[0][2] >= 1 and out[0][1:] == out[1][1:]
+    assert np.array_equal(out[0][0], out[1][0])
