@@ -236,8 +236,8 @@ int pic_job_diagnostics(pic_engine* e, int job, pic_diagnostics* out);
  *   0 = one launch per level (default).  Takes effect at the next field solve.
  * PIC_OPT_MG_CLUSTER_TOP: largest level side solved by a thread-block cluster (65 = none,
  *   default); applies to jobs created after the call.
- * PIC_OPT_MG_COARSE_TOP: largest level side (3..129) solved inside one CTA's shared memory
- *   (65 = default); applies to jobs created after the call.
+ * PIC_OPT_MG_COARSE_TOP: largest level side (3..129) solved inside one CTA (65 = default; with
+ *   the nodes in registers up to 65, in shared memory above); applies to jobs created after the call.
  * PIC_OPT_MOVER_CTAS_PER_SM: warps per SM of the persistent particle pass, in CTAs of 256
  *   threads (0 = as many as fit, the default; larger values are capped there: 28 warps, so 4
  *   and more mean the same as 0).  Takes effect at the next step.

@@ -18,7 +18,7 @@
 // arithmetic and a block barrier per half-sweep, on 1.7 nodes per owned node).  Here a half-sweep
 // of two nodes is one shuffle and six arithmetic instructions, nothing waits at a barrier, and the
 // recomputed halo is 64 / 54 columns: 49 and 99 instructions per node.  Level 0 at 4097^2 (ncu,
-// cold): down 100 -> 40 us (issue 71% active), up 199 -> 131 us (61% of DRAM, 669 MB against 554 MB
+// cold): down 100 -> 40 us (issue 71% active), up 199 -> 131 us (55% of DRAM, 586 MB against 554 MB
 // of inputs and outputs; short and long scoreboard of the shared-memory ring).
 #pragma once
 #include "common.cuh"

@@ -23,8 +23,8 @@
 //   (opt-in: levels up to 257^2 or 513^2 in one thread-block cluster, mg_cluster.cu)
 //   mg_up      prolongation + nu_post sweeps on 32x32 tiles; on level 0 also the FP64
 //              update phi += e, the new FP64 residual and the tile's partial norm;
-//              mg_finish (one CTA per job) adds the partials (mg_norm.cuh: no order matters)
-//              (deterministic), counts the cycle and decides convergence.  The generic
+//              mg_finish (one CTA per job) adds the partials (mg_norm.cuh: exact, in any
+//              order), counts the cycle and decides convergence.  The generic
 //              kernels (mixed smoothing counts) still let the last tile CTA of a job do it.
 #include <algorithm>
 #include "common.cuh"
@@ -959,7 +959,7 @@ __global__ void __launch_bounds__(NT) mg_down_fast_kernel(const TileRef* __restr
 // Up leg (as mg_up_kernel modes 0 and 1).  MODE 0, level l >= 1: the bilinear prolongation
 // of the coarser correction added to the pre-smoothed one, NU post-sweeps, the owned nodes
 // to eu_l.  MODE 1, level 0: the same with a one-node halo, then phi <- phi + e in
-// FP64, the new FP64 defect and the deterministic norm.  The e, f and coarse tiles arrive by
+// FP64, the new FP64 defect and the tile's part of the norm.  The e, f and coarse tiles arrive by
 // tensor-map loads; on level 0 phi64 (with a one-node halo) and rho of the owned nodes come
 // in one batch of asynchronous copies beside them.  MODE 1 on 1024 threads, two CTAs per SM, where level 0
 // has at most wide_factor tiles per SM: its chain of copies, sweeps and the FP64 update is then shorter

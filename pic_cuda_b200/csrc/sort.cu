@@ -52,7 +52,7 @@ __device__ __forceinline__ void run_segment(uint32_t key, int& first, int& last)
 // warp keeps kSortRounds coalesced requests per array in flight.
 constexpr int kSortRounds = 4;
 constexpr int kSortItem = 32 * kSortRounds;
-constexpr int kScatterCtas = 2;   // of the scatter, per SM: all resident at once
+constexpr int kScatterCtas = 2;   // of the scatter, per SM and slot: one slot's are all resident at once
 
 // Histogram of cell keys, one atomic per warp segment of equal keys.  With count_descents, also
 // the particles whose key is below their predecessor's (within a warp iteration's 4 x 32), one
