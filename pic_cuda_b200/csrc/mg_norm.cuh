@@ -22,16 +22,17 @@
 namespace mgn {
 
 __device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }   // -1022 <= e <= 1023
+constexpr int kLeastE2 = -1022;   // u2 is then the least FP64 number: nothing is rounded, no tie to break
 
 // Exponents for a job of side n whose norm's square before the cycle was rnorm2.
 struct Scale {
   int e1, e2;
   __device__ __forceinline__ Scale(double rnorm2, int n) {
     const int e = ((__double2hiint(rnorm2) >> 20) & 0x7ff) - 1023;
-    e1 = min(max(e + 8, -850), 1000);
+    e1 = min(max(e + 8, -1000), 1000);
     // at most 2^bits pairs, whose left-overs of u1 / 2 each make less than 2^62 u2; a lane's 128 fit 2^51 u2
     const int bits = 1 + 2 * (32 - __clz((n + 1) / 2 - 1));
-    e2 = e1 + max(bits - 63, -45);
+    e2 = max(e1 + max(bits - 63, -45), kLeastE2);
   }
 };
 
@@ -45,26 +46,29 @@ static_assert(sizeof(Part) == 16, "two FP64 values of JobDev::partials");
 
 struct Sum {
   double a, b;
-  __device__ __forceinline__ explicit Sum(const Scale& s) : a(1.5 * pow2(s.e1)), b(1.5 * pow2(s.e2)) {}
+  int odd;
+  __device__ __forceinline__ explicit Sum(const Scale& s)
+      : a(1.5 * pow2(s.e1)), b(1.5 * pow2(s.e2)), odd(s.e2 > kLeastE2 ? 1 : 0) {}
   __device__ __forceinline__ void add(double v) {
     const double s = __dadd_rn(a, v), left = __dadd_rn(v, -__dadd_rn(s, -a));
     a = s;
-    b = __dadd_rn(b, __hiloint2double(__double2hiint(left), __double2loint(left) | 1));
+    b = __dadd_rn(b, __hiloint2double(__double2hiint(left), __double2loint(left) | odd));
   }
   // count: the most values that a lane adds.  Left-overs above count u1 / 2 mean that the first part outgrew
   // its exponent; they are kept with it then.
   __device__ __forceinline__ Part part(const Scale& s, int count) const {
     const Sum zero(s);
     const double first = __dadd_rn(a, -zero.a), second = __dadd_rn(b, -zero.b);
-    if (!(fabs(second) <= count * pow2(s.e1 - 53))) return Part{first + second, 0};
-    return Part{first, __double2ll_rn(second * pow2(52 - s.e2))};
+    if (!(fabs(second) <= count * (0x1p-53 * pow2(s.e1)))) return Part{isfinite(first) ? first + second : first, 0};
+    return Part{first, __double2ll_rn(second * pow2(-s.e2) * 0x1p52)};
   }
 };
 // The square of the norm.  The second part gives all its whole u1 to the first, so that one rounding is left.
 __device__ __forceinline__ double total(const Part& p, const Scale& s) {
   const int shift = s.e1 - s.e2;
   const long long whole = (p.second + (1ll << (shift - 1))) >> shift;
-  return __dadd_rn(__dadd_rn(p.first, (double)whole * pow2(s.e1 - 52)), (double)(p.second - (whole << shift)) * pow2(s.e2 - 52));
+  const double rest = (double)(p.second - (whole << shift)) * 0x1p-52 * pow2(s.e2);
+  return __dadd_rn(__dadd_rn(p.first, (double)whole * 0x1p-52 * pow2(s.e1)), rest);
 }
 
 // Squares of a pair's residuals, added.
